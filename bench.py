@@ -111,7 +111,7 @@ def measured_peaks():
 
 def profile_traffic(kernel):
     """dram bytes per launch from the committed ncu summary, if present."""
-    name = {"STEP": "step2d_fused"}.get(kernel, kernel)
+    name = {"STEP": "step2d_block"}.get(kernel, kernel)
     path = os.path.join(ROOT, "profiles", f"{name}_2d_tmz.md")
     try:
         txt = open(path).read()
@@ -501,14 +501,14 @@ def main():
     dft_err = dft_rel_err(jobs32[0], jobs64[0], len(spec32.monitors))
 
     # ---- roofline of the dominant kernel (FP32) ----
-    # with the fused step kernel (the tuner's usual choice here) one launch
-    # per step updates every cell but the dispersive ones, whose kernel runs
-    # beside it; otherwise the interior (core) E and H kernels update nearly
-    # all cells, with the edge and dispersive-cell kernels as parallel branches
+    # with the block-step kernel (the tuner's usual choice here) one launch takes
+    # every cell eight steps on; otherwise the interior (core) E and H kernels
+    # update nearly all cells, with the edge and dispersive-cell kernels as
+    # parallel branches
     if kt32["STEP"][0] > 0:
-        dom, kname, per = "STEP", "step2d_fused (TMz, FP32)", "step"
-        note = ("algorithmic bytes = grid cells x (6w+1): Ez, Hx, Hy read and written once and the material id "
-                "read; the two field sets (~0.2 GB) exceed what stays in the 129 MB L2 between steps")
+        dom, kname, per = "STEP", "step2d_block (TMz, FP32)", "step"
+        note = ("algorithmic bytes = grid cells x (6w+1) per launch of eight steps: Ez, Hx, Hy read and written once "
+                "and the material id read; the kernel is bound by its instructions, not by these bytes")
     else:
         dom = "E" if kt32["E"][1] >= kt32["H"][1] else "H"
         kname, per = f"{dom.lower()}2d_core<float,TM,4>", dom
@@ -558,7 +558,7 @@ def main():
         "vs_baseline": None, "dtype": "f32", "data": "synthetic",
         "config": {"workload": workload_name(args.n, args.nt), "cells": cells, "time_steps_per_job": args.nt,
                    "bench_step": "one job of the workload from a fresh state",
-                   "launch": ("CUDA graph per 32-step ring: the dispersive-cell and fused step kernels per step, "
+                   "launch": ("CUDA graph per 32-step ring: the block-step kernels per eight steps, "
                               "the DFT fold per ring" if kt32["STEP"][0] > 0 else
                               "CUDA graph per 32-step ring (E, H and DFT fold kernels)"),
                    "tile": tile32,

@@ -216,15 +216,29 @@ struct fdtd_job {
   // bounded waits set when they give up
   TmaMaps tma{};
   bool tma_ok = false;
-  // the fused step kernels (FP32): a second set of field buffers Fb (and of
-  // the stored split-PML parts, spb, in 2D), the two sets taking turns as
-  // step n and step n+1 (pp: the set that holds the current step inside
-  // fdtd_step; 0, the canonical F, between calls), and in 3D the tensor maps
-  // of each set's H arrays
+  // the fused 3D step kernel (FP32) and the 2D block-step kernel: a second set
+  // of field buffers Fb (in 2D also of the stored split-PML parts, spb, and of
+  // the dispersive state, ade_b), the two sets taking turns as step n and the
+  // next (pp: the set that holds the current step; settle() brings it back to
+  // the canonical F), and in 3D the tensor maps of each set's H arrays
   bool fused_ok = false;
   void *Fb[6] = {};
-  void *spb[3] = {};
+  void *spb = nullptr;
+  void *ade_b = nullptr;
   int pp = 0;
+  // the 2D block-step kernel's plan: its tiles, their strips' flags and
+  // dispersive cells, and the scratch for state beyond shared memory
+  struct BlockTables {
+    int shape = 0, ks = 0, max_ade = 0, ntiles = 0, ngen = 0, scr_stride = 0;
+    BlockGeom g{};
+    Tile2 *tiles = nullptr;
+    uint16_t *sflags[2] = {};  // of plain and general tiles
+    uint2 *ade = nullptr;
+    void *scratch = nullptr;
+    size_t bytes[5] = {};  // of the five buffers
+  } blk;
+  std::vector<int> ade_cell_host;      // during commit: the dispersive cells and their ids
+  std::vector<uint8_t> ade_mat_host;
   FusedMaps fmaps[2]{};
   int *d_err = nullptr;
   unsigned wait_limit = kWaitLimit;  // polls of a TMA core's mbarrier wait (fdtd_debug_wait_limit)
@@ -577,6 +591,7 @@ int setup_tma(fdtd_job *J);
 int setup_fused(fdtd_job *J);
 
 void free_fused(fdtd_job *J);
+size_t ade_bytes(const fdtd_job *J);
 // the tile (0-based) that selects the fused step kernel
 int fused_tile(const fdtd_job *J) { return J->dim == 3 ? 8 : 3; }
 
@@ -986,6 +1001,8 @@ int commit_impl(fdtd_job *J) {
     ade_cell.push_back((int)c);
     ade_mat.push_back(id);
   }
+  J->ade_cell_host = ade_cell;
+  J->ade_mat_host = ade_mat;
   J->nade = (int)ade_cell.size();
   J->ade_stride = ((J->nade + 31) / 32) * 32;
   if ((rc = alloc_dev(J, (void **)&J->d_ade_cell, sizeof(int) * std::max(1, J->nade)))) return rc;
@@ -1224,6 +1241,8 @@ int commit_impl(fdtd_job *J) {
   if ((rc = setup_fused(J))) return rc;
   if ((rc = tune_tiles<T>(J))) return rc;
   if (J->fused_ok && J->tile != fused_tile(J)) free_fused(J);  // the tuner kept a split shape
+  std::vector<int>().swap(J->ade_cell_host);
+  std::vector<uint8_t>().swap(J->ade_mat_host);
   if ((rc = kernel_flag(J))) return rc;
   J->committed = true;
   return FDTD_OK;
@@ -1288,28 +1307,200 @@ int setup_tma(fdtd_job *J) {
 // The second set of fields (and split parts) of a fused step kernel, with
 // the accounting of its bytes
 void free_fused(fdtd_job *J) {
-  const size_t bytes = (size_t)J->ncell * 4;
+  const size_t bytes = (size_t)J->ncell * J->esz;
   for (int c = 0; c < 6; ++c) { free_dev(J, J->Fb[c], bytes); J->Fb[c] = nullptr; }
-  for (int q = 0; q < 3; ++q) { free_dev(J, J->spb[q], bytes); J->spb[q] = nullptr; }
+  free_dev(J, J->spb, bytes);
+  J->spb = nullptr;
+  free_dev(J, J->ade_b, ade_bytes(J));
+  J->ade_b = nullptr;
+  fdtd_job::BlockTables &B = J->blk;
+  void *const tab[5] = {B.tiles, B.sflags[0], B.sflags[1], B.ade, B.scratch};
+  for (int q = 0; q < 5; ++q) free_dev(J, tab[q], B.bytes[q]);
+  B = fdtd_job::BlockTables{};
   J->fused_ok = false;
 }
 
-// The fused 2D step kernel (TMz, FP32) handles every cell of the grid itself,
-// dispersive cells aside: it needs 4-cell vectors, no periodic axis, no
-// reference slabs, no TFSF box and no mean monitors (the samples are taken
-// in the kernel).  Its second set of Ez, Hx, Hy (and Ezx) is allocated here,
-// before the tuner times the kernel.
-int setup_fused2(fdtd_job *J) {
-  if (J->g.layout != FDTD_LAYOUT_2D_TM || J->esz != 4 || J->vec != 4 || J->g.periodic[0] || J->g.periodic[1] ||
-      J->slab_rows > 0 || J->has_tfbox || !J->gather_fused)
-    return FDTD_OK;
+// bytes of the dispersive state
+size_t ade_bytes(const fdtd_job *J) { return J->esz * (size_t)std::max(1, J->ade_nf) * 3 * std::max(32, J->ade_stride); }
+
+// The tiles of width `len` (o cells owned, h of halo) that hold cell i of an
+// axis of n cells: calls f(tile, place in the tile, whether the tile owns it).
+// On a periodic axis the halo wraps, so a tile may hold images of a cell.
+template <typename F>
+void tiles_of(int i, int n, bool per, int o, int h, int len, F f) {
+  const int nt = (n + o - 1) / o;
+  const int lo = -h, hi = (nt - 1) * o - h + len;  // the span of all tiles
+  const int m0 = per ? -((i - lo) / n) : 0, m1 = per ? (hi - 1 - i) / n : 0;
+  for (int m = m0; m <= m1; ++m) {
+    const int x = i + m * n;
+    if (x < lo || x >= hi) continue;
+    const int t0 = std::max(0, (x + h - len + 1 + o - 1) / o), t1 = std::min(nt - 1, (x + h) / o);
+    for (int t = t0; t <= t1; ++t) {
+      const int l = x - (t * o - h);
+      if (l >= 0 && l < len) f(t, l, m == 0 && l >= h && l < h + o);
+    }
+  }
+}
+
+// The shape and the steps per launch of the 2D block-step kernel.  8 steps: half
+// the launches, loads and stores of 4 for 1.2 times the halo's arithmetic (2048^2
+// with 40 cylinders: 12.3 against 16.9 us a step; 256^2: 2.5 against 4.2).  64-row
+// tiles waste less on the halo, 32-row tiles spread a grid of few tiles over more
+// SMs and leave each half the rows: the line lies where the large ones fill the
+// GPU once (512^2: 2.6 us a step with the small, 4.4 with the large; 1024^2, 220
+// large tiles: 5.5 and 5.3; 2048^2: 15.4 and 12.3).
+void block_choose(const fdtd_job *J, BlockPlan &pl) {
+  pl.ks = kBlockSteps;
+  const BlockShape sh = block_shape(0);
+  const int ox = 32 * sh.V - 2 * ((pl.ks + sh.V - 1) / sh.V * sh.V), oy = sh.RA * sh.NA - 2 * pl.ks;
+  const long long tiles = (long long)((J->nx + ox - 1) / ox) * ((J->ny + oy - 1) / oy);
+  pl.shape = tiles >= J->num_sms ? 0 : 1;
+}
+
+void block_plan(const fdtd_job *J, BlockPlan &pl);
+
+// The plan of the 2D block-step kernel: tiles, the flags of their strips and
+// their dispersive cells; and the second set of buffers.
+// FP32 only: the FP64 arithmetic of the halo costs more than the launches it
+// saves (FP64 runs at 1/64 of the FP32 rate: 256^2 13.2 us a step against 9.3
+// split, 2048^2 116 against 81).
+int setup_block(fdtd_job *J) {
+  typedef float T;
+  if (J->esz != 4 || J->slab_rows > 0 || J->has_tfbox || !J->gather_fused) return FDTD_OK;
   int rc;
-  const size_t bytes = (size_t)J->ncell * 4;
-  for (int c = 2; c <= 4; ++c)
-    if (!J->Fb[c] && (rc = alloc_dev(J, &J->Fb[c], bytes))) return rc;
-  if (J->d_sp[0] && !J->spb[0] && (rc = alloc_dev(J, &J->spb[0], bytes))) return rc;
+  fdtd_job::BlockTables &B = J->blk;
+  BlockPlan pl{};
+  block_choose(J, pl);
+  const BlockShape sh = block_shape(pl.shape);
+  const int W = 32 * sh.V, H = sh.RA * sh.NA;
+  BlockGeom g{};
+  g.nx = J->nx; g.ny = J->ny;
+  g.hy = pl.ks;
+  g.hx = (pl.ks + sh.V - 1) / sh.V * sh.V;
+  g.ox = W - 2 * g.hx;
+  g.oy = H - 2 * g.hy;
+  g.split = J->has_pml && J->pml.mode == FDTD_PML_SPLIT;
+  for (int a = 0; a < 2; ++a) {
+    g.per[a] = J->g.periodic[a];
+    g.slo[a] = J->slo[a]; g.shi[a] = J->shi[a];
+    g.mlo[a] = J->g.main_lo[a]; g.mhi[a] = J->g.main_hi[a];
+  }
+  g.id0 = J->id0;
+  const int ntx = (J->nx + g.ox - 1) / g.ox, nty = (J->ny + g.oy - 1) / g.oy, nt = ntx * nty;
+  std::vector<Tile2> all((size_t)nt), tiles;
+  for (int t = 0; t < nt; ++t)
+    all[t] = Tile2{t % ntx, t / ntx * g.oy, std::min(g.oy, J->ny - t / ntx * g.oy), 0, 0, 0, 0, 0};
+  auto upload = [&](const void *src, void **dst, size_t bytes, int q) -> int {
+    free_dev(J, *dst, B.bytes[q]);
+    *dst = nullptr;
+    B.bytes[q] = bytes;
+    if (const int e = alloc_dev(J, dst, bytes)) return e;
+    if (src) CK(cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice));
+    J->h2d += src ? bytes : 0;
+    return FDTD_OK;
+  };
+  // every tile as a plain one: what its strips hold makes it plain or general
+  if ((rc = upload(all.data(), (void **)&B.tiles, all.size() * sizeof(Tile2), 0))) return rc;
+  if ((rc = upload(nullptr, (void **)&B.sflags[0], (size_t)nt * sh.NA * sizeof(uint16_t), 1))) return rc;
+  launch_tile_flags(J->d_mat, J->d_rowflag, B.tiles, nt, sh.RA, sh.NA, sh.V, g, B.sflags[0], J->stream);
+  CK(cudaGetLastError());
+  CK(cudaStreamSynchronize(J->stream));
+  std::vector<uint16_t> sf((size_t)nt * sh.NA);
+  CK(cudaMemcpy(sf.data(), B.sflags[0], sf.size() * sizeof(uint16_t), cudaMemcpyDeviceToHost));
+  std::vector<char> general((size_t)nt);
+  for (int t = 0; t < nt; ++t) {
+    unsigned f = 0;
+    for (int w = 0; w < sh.NA; ++w) f |= sf[(size_t)t * sh.NA + w] & 0xffu;
+    general[t] = f != 0;
+    all[t].smp = f & SF_SMP ? 1 : 0;
+  }
+  // f(cell, tile, place in the tile, whether the tile owns it) of the dispersive cells
+  auto each = [&](auto f) {
+    for (int q = 0; q < J->nade; ++q) {
+      const int i = J->ade_cell_host[q] % J->nx, j = J->ade_cell_host[q] / J->nx;
+      tiles_of(j, J->ny, g.per[1], g.oy, g.hy, H, [&](int ty, int ly, bool oy) {
+        tiles_of(i, J->nx, g.per[0], g.ox, g.hx, W, [&](int tx, int lx, bool ox) { f(q, ty * ntx + tx, ly * W + lx, ox && oy); });
+      });
+    }
+  };
+  long long total = 0;
+  each([&](int, int t, int, bool) { ++all[t].nade; ++total; });
+  if (total > INT32_MAX) {
+    free_fused(J);
+    return FDTD_OK;  // not offered
+  }
+  // general tiles first, those with the most dispersive cells first among them,
+  // so that no long one starts last
+  std::vector<int> order((size_t)nt);
+  int max_ade = 0, ngen = 0;
+  for (int t = 0; t < nt; ++t) {
+    order[t] = t;
+    max_ade = std::max(max_ade, all[t].nade);
+    ngen += general[t];
+  }
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+    return general[a] != general[b] ? general[a] > general[b] : all[a].nade > all[b].nade;
+  });
+  B.shape = pl.shape; B.ks = pl.ks; B.g = g; B.ntiles = nt; B.ngen = ngen; B.max_ade = max_ade;
+  block_plan(J, pl);
+  std::vector<int> at((size_t)nt);
+  int a0 = 0, s0 = 0;
+  for (int q = 0; q < nt; ++q) {
+    Tile2 &d = all[order[q]];
+    d.ade0 = at[order[q]] = a0;
+    d.scr0 = s0;
+    a0 += d.nade;
+    s0 += std::max(0, d.nade - (d.smp ? pl.cap_smp : pl.cap));
+    tiles.push_back(d);
+  }
+  B.scr_stride = s0;
+  std::vector<uint2> ade((size_t)std::max(1, a0));
+  each([&](int q, int t, int l, bool own) {
+    uint2 e;
+    e.x = (unsigned)q | (own ? 0x80000000u : 0u);
+    e.y = (unsigned)l | (unsigned)J->ade_mat_host[q] << 16;
+    ade[at[t]++] = e;
+  });
+  if (g.per[0] || g.per[1])  // the halo's images come out of order
+    for (const Tile2 &t : tiles)
+      std::sort(ade.begin() + t.ade0, ade.begin() + t.ade0 + t.nade,
+                [](const uint2 &x, const uint2 &y) { return (x.y & 0xffffu) < (y.y & 0xffffu); });
+  if ((rc = upload(tiles.data(), (void **)&B.tiles, tiles.size() * sizeof(Tile2), 0))) return rc;
+  if ((rc = upload(nullptr, (void **)&B.sflags[1], (size_t)std::max(1, ngen) * sh.NB * sizeof(uint16_t), 2))) return rc;
+  launch_tile_flags(J->d_mat, J->d_rowflag, B.tiles + ngen, nt - ngen, sh.RA, sh.NA, sh.V, g, B.sflags[0], J->stream);
+  launch_tile_flags(J->d_mat, J->d_rowflag, B.tiles, ngen, sh.RB, sh.NB, sh.V, g, B.sflags[1], J->stream);
+  CK(cudaGetLastError());
+  if ((rc = upload(ade.data(), (void **)&B.ade, ade.size() * sizeof(uint2), 3))) return rc;
+  if (s0 > 0 &&
+      (rc = upload(nullptr, &B.scratch, (size_t)s0 * J->ade_nf * (J->g.layout == FDTD_LAYOUT_2D_TM ? 1 : 2) * sizeof(T), 4)))
+    return rc;
+  const size_t bytes = (size_t)J->ncell * sizeof(T);
+  for (int c = 0; c < 6; ++c)
+    if (J->F[c] && !J->Fb[c] && (rc = alloc_dev(J, &J->Fb[c], bytes))) return rc;
+  if (J->d_sp[0] && !J->spb && (rc = alloc_dev(J, &J->spb, bytes))) return rc;
+  if (J->nade > 0 && !J->ade_b && (rc = alloc_dev(J, &J->ade_b, ade_bytes(J)))) return rc;
   J->fused_ok = true;
   return FDTD_OK;
+}
+
+// the launch parameters of the job's plan
+void block_plan(const fdtd_job *J, BlockPlan &pl) {
+  const fdtd_job::BlockTables &B = J->blk;
+  pl = BlockPlan{};
+  pl.shape = B.shape;
+  pl.ks = B.ks;
+  pl.nf = J->ade_nf;
+  pl.one_ade = J->ac_host.size() == sizeof(AdeCoef<float>);
+  block_smem(pl, J->g.layout, B.max_ade, B.g.split != 0, !J->mon_dev.empty() || !J->probes.empty());
+  pl.tiles = B.tiles;
+  pl.sflags[0] = B.sflags[0];
+  pl.sflags[1] = B.sflags[1];
+  pl.ngen = B.ngen;
+  pl.ade = B.ade;
+  pl.g = B.g;
+  pl.ntiles = B.ntiles;
+  pl.scratch = (float *)B.scratch;
+  pl.scr_stride = B.scr_stride;
 }
 
 // The fused 3D step kernel needs what the TMA cores need on both sides of the
@@ -1320,7 +1511,8 @@ int setup_fused2(fdtd_job *J) {
 int setup_fused(fdtd_job *J) {
   J->fused_ok = false;
   if (getenv("FDTD_NO_FUSED") || J->ncore <= 0) return FDTD_OK;
-  if (J->dim == 2) return setup_fused2(J);
+  if (J->tile_req > 0 && J->tile_req != fused_tile(J) + 1) return FDTD_OK;  // another shape is pinned
+  if (J->dim == 2) return setup_block(J);
   if (J->dim != 3 || !J->tma_ok || !J->tma.h_ok || J->slab_rows > 0 || J->has_tfbox) return FDTD_OK;
   PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
   if (!enc) return FDTD_OK;
@@ -1465,7 +1657,7 @@ void fill_common(fdtd_job *J, StepParams<T> &p) {
 template <typename T>
 void ring_params(fdtd_job *J, StepParams<T> &p, bool graph) {
   p.d_base = graph ? J->d_base : nullptr;
-  if (graph) {
+  if (graph && J->d_half) {  // (a pack's ring stays in the job's current half)
     p.stage = (T *)J->d_stage;
     p.d_half = J->d_half;
   }
@@ -1710,6 +1902,40 @@ int run_parts(fdtd_job *J, const StepParams<T> &p, const bool (&want)[3], bool e
 std::mutex g_tune_mu;
 std::map<long long, int> g_tune;
 
+// the block-step launch's two sets of buffers: step n in set `from`, the new
+// step to the other
+void block_buffers(const fdtd_job *J, StepParams<float> &p, BlockPlan &pl, int from) {
+  float *A[6], *B[6];
+  for (int c = 0; c < 6; ++c) {
+    A[c] = (float *)(from ? J->Fb[c] : J->F[c]);
+    B[c] = (float *)(from ? J->F[c] : J->Fb[c]);
+  }
+  p.ex = A[0]; p.ey = A[1]; p.ez = A[2]; p.hx = A[3]; p.hy = A[4]; p.hz = A[5];
+  p.exo = B[0]; p.eyo = B[1]; p.ezo = B[2]; p.hxo = B[3]; p.hyo = B[4]; p.hzo = B[5];
+  p.sp[0] = (float *)(from ? J->spb : J->d_sp[0]);
+  p.spo = (float *)(from ? J->d_sp[0] : J->spb);
+  p.ade_state = (float *)(from ? J->ade_b : J->d_ade_state);
+  pl.ade_out = (float *)(from ? J->d_ade_state : J->ade_b);
+  p.pp = 1;
+}
+
+// The tiles of a block-step launch: general and plain ones write different
+// cells, so their two kernels run beside one another, the plain one on a side
+// stream.  Returns the kernels launched, -1 on failure.
+int launch_blocks(fdtd_job *J, const StepParams<float> &p, const BlockPlan &pl) {
+  const bool both = pl.ngen > 0 && pl.ngen < pl.ntiles && !J->prof;
+  if (!both) return launch_step2d_block(p, pl, true, J->stream) + launch_step2d_block(p, pl, false, J->stream);
+  auto ok = [](cudaError_t e) {
+    if (e != cudaSuccess) set_err(FDTD_ECUDA, "block-step launch: %s", cudaGetErrorString(e));
+    return e == cudaSuccess;
+  };
+  if (!ok(cudaEventRecord(J->ev_fork, J->stream)) || !ok(cudaStreamWaitEvent(J->side[0], J->ev_fork, 0))) return -1;
+  int n = launch_step2d_block(p, pl, true, J->stream);
+  n += launch_step2d_block(p, pl, false, J->side[0]);
+  if (!ok(cudaEventRecord(J->ev_join[0], J->side[0])) || !ok(cudaStreamWaitEvent(J->stream, J->ev_join[0], 0))) return -1;
+  return n;
+}
+
 template <typename T>
 int tune_tiles(fdtd_job *J) {
   if (J->dim < 2 || J->ncore <= 0) return FDTD_OK;
@@ -1720,8 +1946,9 @@ int tune_tiles(fdtd_job *J) {
     if (J->dim == 3 && J->tile == 8 && !J->fused_ok)
       return set_err(FDTD_EINVAL, "tile 9 (the fused step kernel) needs FP32, 4-cell vectors, a core box inside the "
                                   "grid, and no reference slabs or TFSF box");
-    if (J->dim == 2 && J->tile == 3 && !J->fused_ok)
-      return set_err(FDTD_EINVAL, "2D tile 4 (the fused step kernel) needs TMz, FP32, nx a multiple of 4, no periodic "
+    if (J->dim == 2 && J->tile == 3 &&
+        (!J->fused_ok || J->g.layout != FDTD_LAYOUT_2D_TM || J->esz != 4 || J->vec != 4 || J->g.periodic[0] || J->g.periodic[1]))
+      return set_err(FDTD_EINVAL, "2D tile 4 (the block-step kernel) needs TMz, FP32, nx a multiple of 4, no periodic "
                                   "axis, and no reference slabs, TFSF box or mean monitors");
     return FDTD_OK;
   }
@@ -1732,8 +1959,12 @@ int tune_tiles(fdtd_job *J) {
   }
   int lg = 0;
   for (long long c = J->ncore; c > 1; c >>= 1) ++lg;
-  // which TMA-staged kernels the grid can take is part of the kind of grid
-  const long long key = (((((long long)J->dim * 8 + J->g.layout) * 4 + J->g.precision) * 8 + J->vec) * 64 + lg) * 8 +
+  // which TMA-staged kernels the grid can take, and the share of dispersive
+  // cells (halvings, up to 15), are part of the kind of grid
+  int lade = 0;
+  for (long long c = J->nade; lade < 15 && c < J->ncore; c *= 2, ++lade)
+    if (c == 0) { lade = 15; break; }
+  const long long key = ((((((long long)J->dim * 8 + J->g.layout) * 4 + J->g.precision) * 8 + J->vec) * 64 + lg) * 16 + lade) * 8 +
                         (J->fused_ok ? 4 : 0) + (J->tma_ok ? 2 : 0) + (J->tma_ok && J->tma.h_ok ? 1 : 0);
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
@@ -1757,30 +1988,51 @@ int tune_tiles(fdtd_job *J) {
   // step the edge and dispersive-cell kernels run beside the cores, and
   // their work is a small part of a grid large enough for the fused kernel)
   const int nshapes = J->dim == 3 ? (J->fused_ok ? 9 : J->tma_ok ? (J->tma.h_ok ? 8 : 7) : 6) : J->fused_ok ? 4 : 3;
+  // 2D: the block-step kernel takes whole steps, so it is timed against the
+  // whole split step of the best core shape: cores, edge and dispersive cells
+  BlockPlan pl{};
+  if (J->dim == 2 && J->fused_ok) block_plan(J, pl);
+  auto split_step = [&] {
+    const bool parts[3] = {true, true, false};
+    p.roles = ROLE_MAIN | ROLE_PML | ROLE_ADE;
+    p.tile = choice;
+    run_parts<T>(J, p, parts, true, true);
+    run_parts<T>(J, p, parts, false, true);
+  };
   auto cores = [&](int c) {
     if constexpr (sizeof(T) == 4) {
-      if (c == fused_tile(J)) {
+      if (J->dim == 2 && c == fused_tile(J)) {
+        StepParams<float> q = p;
+        block_buffers(J, q, pl, 0);
+        launch_blocks(J, q, pl);
+        return;
+      }
+      if (J->dim == 3 && c == fused_tile(J)) {
         StepParams<float> q = p;
         q.exo = (float *)J->Fb[0]; q.eyo = (float *)J->Fb[1]; q.ezo = (float *)J->Fb[2];
         q.hxo = (float *)J->Fb[3]; q.hyo = (float *)J->Fb[4]; q.hzo = (float *)J->Fb[5];
-        q.spo[0] = (float *)J->spb[0];
         q.pp = 1;
-        if (J->dim == 3) launch_step3d_fused(q, J->fmaps[0], J->stream);
-        else launch_step2d_fused(q, J->stream);
+        launch_step3d_fused(q, J->fmaps[0], J->stream);
         return;
       }
     }
     launch_part<T>(J, p, K2D_CORE, true, J->stream);
     launch_part<T>(J, p, K2D_CORE, false, J->stream);
   };
-  for (int c = 0; c < nshapes; ++c) {
-    p.tile = c;
-    for (int w = 0; w < 2; ++w) cores(c);
+  auto time5 = [&](auto run) {
+    for (int w = 0; w < 2; ++w) run();
     cudaEventRecord(a, J->stream);
-    for (int r = 0; r < 5; ++r) cores(c);
+    for (int r = 0; r < 5; ++r) run();
     cudaEventRecord(b, J->stream);
     float ms = 0.f;
-    if (cudaEventSynchronize(b) == cudaSuccess && cudaEventElapsedTime(&ms, a, b) == cudaSuccess && ms < best) {
+    return cudaEventSynchronize(b) == cudaSuccess && cudaEventElapsedTime(&ms, a, b) == cudaSuccess ? ms : 3.0e38f;
+  };
+  for (int c = 0; c < nshapes; ++c) {
+    const bool block = J->dim == 2 && c == fused_tile(J);
+    if (block) best = time5(split_step);
+    p.tile = c;
+    const float ms = time5([&] { cores(c); }) / (block ? (float)pl.ks : 1.f);  // of a step
+    if (ms < best) {
       best = ms;
       choice = c;
     }
@@ -1863,18 +2115,9 @@ int after_sample(fdtd_job *J, int n) {
 // chose it.  The per-procedure entry points keep the split kernels.
 bool fused_mode(const fdtd_job *J) { return J->fused_ok && J->tile == fused_tile(J); }
 
-// One time step of the fused 2D path, from field set pp to the other: the
-// dispersive cells' E (E^n and H^n of the current set, E^{n+1} into the
-// other), then the fused kernel over the whole grid, which takes the samples
-// of the new fields itself.  The fused kernel follows e2d_ade with a
-// programmatic dependency and waits for it only at dispersive cells.
-int fused_step2(fdtd_job *J, int n, int slot, bool graph) {
-  const int from = J->pp, to = 1 - from;
-  float *A[6] = {}, *B[6] = {};
-  for (int c = 0; c < 6; ++c) {
-    A[c] = (float *)(from ? J->Fb[c] : J->F[c]);
-    B[c] = (float *)(to ? J->Fb[c] : J->F[c]);
-  }
+// k steps (at most the plan's) of the 2D block-step kernel in one launch, from
+// field set pp to the other; it takes the samples of each step itself.
+int block_step(fdtd_job *J, int n, int k, int slot, bool graph) {
   StepParams<float> p;
   fill_common<float>(J, p);
   set_sources<float>(J, p);
@@ -1883,18 +2126,16 @@ int fused_step2(fdtd_job *J, int n, int slot, bool graph) {
   p.slot = slot;
   ring_params(J, p, graph);
   p.gather = 1;
-  p.pp = 1;
-  p.ez = A[2]; p.hx = A[3]; p.hy = A[4];
-  p.ezo = B[2]; p.hxo = B[3]; p.hyo = B[4];
-  p.sp[0] = (float *)(from ? J->spb[0] : J->d_sp[0]);
-  p.spo[0] = (float *)(to ? J->spb[0] : J->d_sp[0]);
-  if (!graph) ev_record(J, FDTD_KERNEL_ADE, true);
-  J->launches += launch_e2d_ade_pdl<float>(p, J->stream);
-  if (!graph) ev_record(J, FDTD_KERNEL_ADE, false);
+  BlockPlan pl;
+  block_plan(J, pl);
+  pl.ks = k;
+  block_buffers(J, p, pl, J->pp);
   if (!graph) ev_record(J, FDTD_KERNEL_STEP, true);
-  J->launches += launch_step2d_fused(p, J->stream);
+  const int ran = launch_blocks(J, p, pl);
   if (!graph) ev_record(J, FDTD_KERNEL_STEP, false);
-  J->pp = to;
+  if (ran < 0) return FDTD_ECUDA;
+  J->launches += ran;
+  J->pp ^= 1;
   J->prog_prev = -1;
   CK(cudaGetLastError());
   return FDTD_OK;
@@ -1912,7 +2153,6 @@ int fused_step(fdtd_job *J, int n, int slot, bool graph) {
     (void)n; (void)slot; (void)graph;
     return set_err(FDTD_ESTATE, "the fused step kernel is FP32 only");
   } else {
-    if (J->dim == 2) return fused_step2(J, n, slot, graph);
     const int from = J->pp, to = 1 - from;
     float *A[6], *B[6];
     for (int c = 0; c < 6; ++c) {
@@ -1954,24 +2194,34 @@ int fused_step(fdtd_job *J, int n, int slot, bool graph) {
   }
 }
 
-// After an odd number of fused steps the current fields are in the second
-// set: copy them to the canonical one, where every other entry point and the
-// ring graph (which starts from it) expect them.
+// After an odd number of launches over the two sets the current fields are in
+// the second one: copy them to the canonical one, where every entry point but
+// fdtd_step, and the ring graph (which starts from it), expect them.
 int fused_settle(fdtd_job *J) {
   if (!J->pp) return FDTD_OK;
-  const size_t bytes = (size_t)J->ncell * 4;
+  const size_t bytes = (size_t)J->ncell * J->esz;
   for (int c = 0; c < 6; ++c)
     if (J->Fb[c]) CK(cudaMemcpyAsync(J->F[c], J->Fb[c], bytes, cudaMemcpyDeviceToDevice, J->stream));
-  for (int q = 0; q < 3; ++q)
-    if (J->spb[q]) CK(cudaMemcpyAsync(J->d_sp[q], J->spb[q], bytes, cudaMemcpyDeviceToDevice, J->stream));
+  if (J->spb) CK(cudaMemcpyAsync(J->d_sp[0], J->spb, bytes, cudaMemcpyDeviceToDevice, J->stream));
+  if (J->ade_b) CK(cudaMemcpyAsync(J->d_ade_state, J->ade_b, ade_bytes(J), cudaMemcpyDeviceToDevice, J->stream));
   J->pp = 0;
   J->prog_prev = -1;
   return FDTD_OK;
 }
 
+// Steps n.. of the eager path, at most `left` of them; *done: how many ran.
 template <typename T>
-int eager_step(fdtd_job *J, int n) {
+int eager_steps(fdtd_job *J, int n, int left, int *done) {
   int rc;
+  *done = 1;
+  if (fused_mode(J) && J->dim == 2) {  // as many as a launch takes and the sample ring has room for
+    const int k = std::min(std::min(left, J->blk.ks), kStageSteps - J->stage_fill);
+    if ((rc = block_step(J, n, k, J->stage_fill, false))) return rc;
+    for (int s = 0; s < k; ++s)
+      if ((rc = after_sample<T>(J, n + s))) return rc;
+    *done = k;
+    return FDTD_OK;
+  }
   if (fused_mode(J)) {
     if ((rc = fused_step<T>(J, n, J->stage_fill, false))) return rc;
     return after_sample<T>(J, n);
@@ -2024,9 +2274,14 @@ int ring_graph(fdtd_job *J) {
     }
     if (bad) bad = set_err(FDTD_ECUDA, "fold branch of the ring graph");
   }
-  // the fused path alternates the field sets over the ring's even number of
-  // steps, so a replay starts and ends with the canonical set
+  // the fused and block paths alternate the field sets over the ring's even
+  // number of launches, so a replay starts and ends with the canonical set
   for (int s = 0; s < kStageSteps && !bad; ++s) {
+    if (fused_mode(J) && J->dim == 2) {
+      bad = block_step(J, 0, J->blk.ks, s, true);
+      s += J->blk.ks - 1;
+      continue;
+    }
     if (fused_mode(J)) {
       bad = fused_step<T>(J, 0, s, true);
       continue;
@@ -2196,8 +2451,9 @@ int step_impl(fdtd_job *J, int n_first, int n_steps) {
   int n = n_first;
   // finish a partly filled ring eagerly, replay whole rings from the graph,
   // run the tail eagerly (the per-launch events of fdtd_profile need eager)
-  while (n < end && J->stage_fill != 0)
-    if ((rc = eager_step<T>(J, n++))) return rc;
+  int k = 0;
+  for (; n < end && J->stage_fill != 0; n += k)
+    if ((rc = eager_steps<T>(J, n, end - n, &k))) return rc;
   if (J->use_graph && !J->prof && end - n >= kStageSteps) {
     if ((rc = fused_settle(J))) return rc;
     while (end - n >= kStageSteps) {
@@ -2206,9 +2462,9 @@ int step_impl(fdtd_job *J, int n_first, int n_steps) {
     }
     if ((rc = flush_fold<T>(J))) return rc;
   }
-  while (n < end)
-    if ((rc = eager_step<T>(J, n++))) return rc;
-  return fused_settle(J);
+  for (; n < end; n += k)
+    if ((rc = eager_steps<T>(J, n, end - n, &k))) return rc;
+  return J->dim == 3 ? fused_settle(J) : FDTD_OK;
 }
 
 #define DISPATCH(J, call) ((J)->g.precision == FDTD_F32 ? call<float> : call<double>)
@@ -2227,6 +2483,7 @@ static int proc_call(fdtd_job *J, int n, int what) {
   int rc = ensure_probe_cap(J, n);
   if (rc) return rc;
   if (J->dim >= 2 && (rc = ensure_srctab(J, n))) return rc;
+  if ((rc = fused_settle(J))) return rc;
   if (J->dim == 1) {
     if (what == 0) { if (J->stage_fill == 0) J->stage_n0 = n; return line_run<T>(J, n, 1, ST_E); }
     if (what == 2) return line_run<T>(J, n, 1, ST_H);
@@ -2260,6 +2517,7 @@ template <typename T>
 static int get_field_impl(fdtd_job *J, int comp, double *host) {
   if (comp < 0 || comp > 7 || !J->F[comp]) return set_err(FDTD_EINVAL, "component %d not in this layout", comp);
   const long long cnt = field_elems(J, comp);
+  if (const int rc = fused_settle(J)) return rc;
   std::vector<T> tmp((size_t)cnt);
   CK(cudaMemcpyAsync(tmp.data(), J->F[comp], (size_t)cnt * sizeof(T), cudaMemcpyDeviceToHost, J->stream));
   CK(cudaStreamSynchronize(J->stream));
@@ -2272,6 +2530,7 @@ template <typename T>
 static int set_field_impl(fdtd_job *J, int comp, const double *host) {
   if (comp < 0 || comp > 7 || !J->F[comp]) return set_err(FDTD_EINVAL, "component %d not in this layout", comp);
   const long long cnt = field_elems(J, comp);
+  if (const int rc = fused_settle(J)) return rc;
   std::vector<T> tmp(host, host + cnt);
   CK(cudaMemcpyAsync(J->F[comp], tmp.data(), (size_t)cnt * sizeof(T), cudaMemcpyHostToDevice, J->stream));
   CK(cudaStreamSynchronize(J->stream));
@@ -2411,11 +2670,67 @@ int pack_capture(fdtd::Pack *P) {
   return FDTD_OK;
 }
 
+// A pack of jobs that run the block-step kernel: each job's launches of a ring,
+// and the fold of its samples, are a branch of the ring's graph.  (Their tiles
+// fill the GPU from several branches at once: 16 jobs of 256^2 ran at 44
+// Gcell/s as concurrent launches, at 29 through the shared half-step launches.)
+int pack_capture_blocks(fdtd::Pack *P) {
+  const int nj = (int)P->jobs.size();
+  int kernels = 0;
+  cudaError_t bad = cudaStreamBeginCapture(P->stream, cudaStreamCaptureModeThreadLocal);
+  if (bad != cudaSuccess) return set_err(FDTD_ECUDA, "pack graph capture: %s", cudaGetErrorString(bad));
+  int rc = FDTD_OK;
+  bad = cudaEventRecord(P->ev_fork, P->stream);
+  for (int q = 0; q < nj && bad == cudaSuccess && !rc; ++q) {
+    fdtd_job *J = P->jobs[q];
+    // the job's own stream and events carry its branch during the capture
+    int *const own_base = J->d_base, *const own_half = J->d_half;
+    const long long launches0 = J->launches;
+    bad = cudaStreamWaitEvent(J->stream, P->ev_fork, 0);
+    J->d_base = P->d_n0 + q;
+    J->d_half = nullptr;
+    J->prog_prev = -1;
+    for (int s = 0; s < kStageSteps && !rc && bad == cudaSuccess; s += J->blk.ks)
+      rc = block_step(J, 0, J->blk.ks, s, true);
+    if (!rc && bad == cudaSuccess && !J->mon_dev.empty() && J->dft_blocks > 0) {
+      DftParams d;
+      fold_params(J, d);
+      d.nslots = kStageSteps;
+      d.d_base = P->d_n0 + q;
+      launch_dft<float>(d, (const float *)J->d_stage + (size_t)J->stage_half * kStageSteps * J->stage_row, J->stream);
+      J->launches++;
+      bad = cudaGetLastError();
+    }
+    if (bad == cudaSuccess) bad = cudaEventRecord(J->ev_fjoin, J->stream);
+    if (bad == cudaSuccess) bad = cudaStreamWaitEvent(P->stream, J->ev_fjoin, 0);
+    kernels += (int)(J->launches - launches0);
+    J->launches = launches0;
+    J->d_base = own_base;
+    J->d_half = own_half;
+    J->prog_prev = -1;
+  }
+  if (bad == cudaSuccess && !rc) {
+    pack_advance_kernel<<<(nj + 31) / 32, 32, 0, P->stream>>>(P->d_n0, nj, kStageSteps);
+    ++kernels;
+    bad = cudaGetLastError();
+  }
+  cudaGraph_t g = nullptr;
+  const cudaError_t e = cudaStreamEndCapture(P->stream, &g);
+  if (rc || bad != cudaSuccess || e != cudaSuccess) {
+    if (g) cudaGraphDestroy(g);
+    return rc ? rc : set_err(FDTD_ECUDA, "pack graph capture: %s", cudaGetErrorString(bad != cudaSuccess ? bad : e));
+  }
+  P->graph = g;
+  CK(cudaGraphInstantiate(&P->exec, P->graph, 0));
+  P->kernels_per_ring = kernels;
+  return FDTD_OK;
+}
+
 }  // namespace
 
 long long fdtd::pack_key(const fdtd_job *J) {
   if (!J || !J->committed || J->dim != 2 || !J->gather_fused || J->prof || J->stage_fill != 0) return -1;
-  return ((long long)J->g.precision * 16 + J->g.layout) * 16 + J->vec;
+  return (((long long)J->g.precision * 16 + J->g.layout) * 16 + J->vec) * 2 + (fused_mode(J) ? 1 : 0);
 }
 
 int fdtd::job_reserve(fdtd_job *J, int n_last) {
@@ -2459,7 +2774,8 @@ int fdtd::pack_create(fdtd_job *const *jobs, int njobs, fdtd::Pack **out) {
          cudaEventCreateWithFlags(&P->ev_join[q], cudaEventDisableTiming) == cudaSuccess;
   std::vector<int> n0(njobs);
   for (int q = 0; q < njobs && ok; ++q) {
-    ok = cudaStreamSynchronize(jobs[q]->stream) == cudaSuccess;  // the job's own work is done
+    // the job's own work is done, its fields in the canonical buffers
+    ok = fused_settle(jobs[q]) == FDTD_OK && cudaStreamSynchronize(jobs[q]->stream) == cudaSuccess;
     n0[q] = jobs[q]->last_n + 1;
   }
   if (ok) ok = cudaMallocAsync((void **)&P->d_n0, njobs * sizeof(int), P->stream) == cudaSuccess &&
@@ -2469,7 +2785,7 @@ int fdtd::pack_create(fdtd_job *const *jobs, int njobs, fdtd::Pack **out) {
     pack_destroy(P);
     return set_err(FDTD_ECUDA, "pack set-up failed");
   }
-  const int rc = P->f64 ? pack_capture<double>(P) : pack_capture<float>(P);
+  const int rc = fused_mode(jobs[0]) ? pack_capture_blocks(P) : P->f64 ? pack_capture<double>(P) : pack_capture<float>(P);
   if (rc) {
     pack_destroy(P);
     return rc;
@@ -2823,6 +3139,7 @@ int fdtd_check_finite(fdtd_job *J, int64_t *count) {
   int rc = check_job(J, true);
   if (rc) return rc;
   if (!count) return set_err(FDTD_EINVAL, "null count");
+  if ((rc = fused_settle(J))) return rc;
   if (!J->d_count && (rc = alloc_dev(J, (void **)&J->d_count, sizeof(unsigned long long)))) return rc;
   CK(cudaMemsetAsync(J->d_count, 0, sizeof(unsigned long long), J->stream));
   for (auto &s : J->state)
@@ -2893,6 +3210,7 @@ int fdtd_save_state(fdtd_job *J, void *buf, uint64_t bytes) {
   if (bytes < need) return set_err(FDTD_ERANGE, "checkpoint needs %llu bytes, got %llu", (unsigned long long)need,
                                    (unsigned long long)bytes);
   // the step boundary: everything queued has run; the ring is not folded
+  if ((rc = fused_settle(J))) return rc;
   CK(cudaStreamSynchronize(J->stream));
   CK(cudaGetLastError());
   char *o = (char *)buf;
@@ -2977,6 +3295,7 @@ int fdtd_load_state(fdtd_job *J, const void *buf, uint64_t bytes) {
   if (expect != bytes) return set_err(FDTD_EINVAL, "checkpoint of %llu bytes, its tables describe %llu",
                                       (unsigned long long)bytes, (unsigned long long)expect);
   CK(cudaStreamSynchronize(J->stream));
+  J->pp = 0;  // the loaded state goes to the canonical buffers
   if (n_probe_max > 0 && (rc = ensure_probe_cap(J, n_probe_max))) return rc;
   const char *o = pr + J->probes.size() * 2 * sizeof(int32_t);
   for (auto &s : J->state) {
@@ -3108,10 +3427,10 @@ int fdtd_estimate_bytes(const fdtd_job *J, uint64_t *bytes) {
   if (J->dim == 3 && w == 4 && J->nx % 4 == 0 && !J->has_tfbox &&
       !(J->has_pml && J->pml.mode == FDTD_PML_REFERENCE))
     b += 6 * N * w;
-  // the fused 2D step kernel's: Ez, Hx, Hy and the stored PML part
-  if (J->g.layout == FDTD_LAYOUT_2D_TM && w == 4 && J->nx % 4 == 0 && !J->has_tfbox &&
-      !(J->has_pml && J->pml.mode == FDTD_PML_REFERENCE))
-    b += 4 * N * w;
+  // the 2D block-step kernel's: the fields and the stored PML part, its tiles
+  // (at least 112 x 16 cells, 96 bytes with their flags)
+  const bool block2 = J->dim == 2 && w == 4 && !J->has_tfbox && !(J->has_pml && J->pml.mode == FDTD_PML_REFERENCE);
+  if (block2) b += 4 * N * w + ((uint64_t)nx / 112 + 1) * ((uint64_t)ny / 16 + 1) * 96;
   if (J->has_tfsf) b += 2 * N * w;
   if (J->has_tfbox) b += 2ull * ny * w + 4 * w;
   // dispersive cells: each region's cells, bounded per sphere / box
@@ -3140,6 +3459,9 @@ int fdtd_estimate_bytes(const fdtd_job *J, uint64_t *bytes) {
   for (auto &m : J->mats) nf = std::max(nf, ade_fields(m.kind, m.lz.npoles, m.lz.chi3 != 0.0, m.lz.ez_uses_x_current != 0));
   nf = std::max(nf, 1);
   b += nade * ((uint64_t)nf * 3 * w + 5) + 32ull * nf * 3 * w;
+  // and its dispersive cells: a second state, and in up to four tiles a list
+  // entry and the scratch state
+  if (block2) b += nade * ((uint64_t)nf * 3 * w + 4 * (8 + 2ull * nf * w)) + 32ull * nf * 3 * w;
   if (J->has_pml && J->pml.mode == FDTD_PML_SPLIT) {
     b += (uint64_t)(J->dim == 3 ? 6 : 1) * (w == 8 ? 2 : 1) * N * w;
     b += 4ull * (nx + ny + nz) * w;

@@ -176,8 +176,8 @@ struct StepParams {
                            // 2D TM: Ezx; 2D TE: Hzx).  FP64 also stores the
                            // other parts in sp[6+q] (Exz Eyx Ezy Hxz Hyx Hzy /
                            // Ezy / Hzy); FP32 takes them as total - part.
-  T *spo[3];               // the fused 2D step: where sp[0..2] of step n+1 go
-                           // (the other buffer of a ping-pong pair)
+  T *spo;                  // the 2D block-step kernel: where sp[0] of the new step goes (the
+                           // other buffer of a ping-pong pair)
   // reference y-slabs (2D: Ex Ey Hzx Hzy; 3D: 12 split arrays) per side
   int slab_on[2];
   int slab_j0[2];          // first 0-based row of the slab
@@ -263,13 +263,63 @@ enum K2dPart { K2D_CORE = 0, K2D_EDGE = 1, K2D_ADE = 2 };
 // prog_event: the core kernel records it as a programmatic event (or null)
 template <typename T> int launch_e2d(const StepParams<T> &p, int part, void *stream, void *prog_event = nullptr);
 
-// the dispersive cells' E update with a programmatic dependency on the kernel
-// before it (the first launch of a fused 2D step); returns the kernels launched
-template <typename T> int launch_e2d_ade_pdl(const StepParams<T> &p, void *stream);
-// the fused 2D step kernel (k2f.cu, TMz, FP32): E^{n+1} and H^{n+1} of every
-// cell in one pass, reading ez, hx, hy, sp[0] and storing to ezo, hxo, hyo,
-// spo[0]; returns the kernels launched
-int launch_step2d_fused(const StepParams<float> &p, void *stream);
+// ---- the 2D block-step kernel (k2b.cu, FP32) ------------------------------------
+// A block's tile: column tx, rows y0.. (oy owned), its dispersive cells (its part
+// of BlockPlan::ade) and the first of its entries in the scratch buffer for
+// their state.
+struct Tile2 {
+  int tx, y0, oy;
+  int ade0, nade;
+  int scr0;
+  int smp;      // it may hold rows with samples
+  int pad;
+};
+// flags of a tile's warp strips: cells that are not main cells, main cells of
+// several materials or dispersive ones, rows with a source, rows with a sample,
+// split-PML cells
+enum StripFlag : int { SF_GEN = 1, SF_MIX = 2, SF_SRC = 4, SF_SMP = 8, SF_SHELL = 16 };
+// tiles of ox cells by oy rows, widened by hx cells and hy rows
+struct BlockGeom {
+  int nx, ny;
+  int ox, oy, hx, hy;
+  int per[2];
+  int split;
+  int slo[2], shi[2], mlo[2], mhi[2];
+  int id0;
+};
+struct BlockPlan {
+  const Tile2 *tiles;     // the general ones (any cells, sources, samples) first
+  int ngen;
+  const uint16_t *sflags[2];  // plain, general: per tile and warp StripFlag bits, material id << 8
+  const uint2 *ade;       // x: slot, bit 31: the tile owns the cell; y: cell in the tile, material id << 16
+  BlockGeom g;
+  int ntiles;
+  int shape;              // kernel shape (BlockShape)
+  int ks;                 // steps of this launch, at most hy
+  int one_ade;            // every dispersive cell is of the first dispersive material
+  int nf;                 // state fields of a dispersive cell
+  int cap, cap_smp;       // dispersive cells of a tile whose state fits in shared memory (of one with samples)
+  int off_crv, off_st, off_smp;  // byte offsets in dynamic shared memory
+  int smem;               // its bytes
+  float *scratch;         // state beyond cap, [field][component][scr_stride]
+  int scr_stride;
+  float *ade_out;         // the other set of the dispersive state
+};
+// one shape of the kernel: V cells per thread along x; plain tiles: RA rows per
+// warp and NA warps, general ones RB and NB (the same rows in all)
+struct BlockShape {
+  int V, RA, NA, RB, NB;
+};
+constexpr int kBlockShapes = 2;
+constexpr int kBlockSteps = 8;  // most steps of a launch
+BlockShape block_shape(int shape);
+// bytes of dynamic shared memory (and the plan's offsets) for tiles with at
+// most max_ade dispersive cells; sets cap
+void block_smem(BlockPlan &pl, int layout, int max_ade, bool split, bool smp_rows);
+// the general or the plain tiles of a launch; returns the kernels launched
+int launch_step2d_block(const StepParams<float> &p, const BlockPlan &pl, bool gen, void *stream);
+void launch_tile_flags(const uint8_t *mat, const uint8_t *rowflag, const Tile2 *tiles, int ntiles, int R, int NW, int V,
+                       const BlockGeom &g, uint16_t *out, void *stream);
 
 // packs of 2D jobs: one launch runs one part of every job's half step
 constexpr int kMaxPack = 32;

@@ -16,7 +16,8 @@
 //   ADE  : one thread per dispersive cell (gold Drude+2CP,
 //          2D/gold_mod.f90:47-75); core and edge threads never store E there.
 //          Its blocks follow the edge units' in the E edge launch
-//          (e2d_edge_ade); the fused 2D step launches them alone (e2d_ade).
+//          (e2d_edge_ade).
+// FP32 jobs mostly run whole steps in the block-step kernel instead (k2b.cu).
 #include <cuda_runtime.h>
 
 #include "fdtd_internal.h"
@@ -326,7 +327,7 @@ struct K2 {
 #pragma unroll
         for (int q = 0; q < V; ++q) {
           const T vals[6] = {T(0), T(0), cur[q], h0[q], h1[q], T(0)};
-          gather_cell<T>(p, n, i0 + q, j, 0, vals);
+          gather_cell<T>(p, n, i0 + q, j, 0, vals, p.slot);
         }
       }
     } else {
@@ -392,7 +393,7 @@ struct K2 {
 #pragma unroll
         for (int q = 0; q < V; ++q) {
           const T vals[6] = {cur[q], xe[q], T(0), T(0), T(0), h0[q]};
-          gather_cell<T>(p, n, i0 + q, j, 0, vals);
+          gather_cell<T>(p, n, i0 + q, j, 0, vals, p.slot);
         }
       }
     }
@@ -583,30 +584,6 @@ __global__ void __launch_bounds__(256) h2d_edge(const __grid_constant__ StepPara
   K2<T, L, V>::unit_h(p, __ldg(p.edge_units + t), step_n(p));
 }
 
-// The fused 2D step kernel follows this one with a programmatic dependency
-// and waits for it only where it meets a dispersive cell: it may start once
-// every block here has passed its own wait (and with it, the previous step).
-template <typename T, int L, int KIND>
-__global__ void __launch_bounds__(256) e2d_ade(const __grid_constant__ StepParams<T> p) {
-  pdl_wait();
-  pdl_release();
-  const int s = blockIdx.x * 256 + threadIdx.x;
-  if (s < p.nade) ade_e2<T, L, KIND>(p, s, step_n(p));
-}
-
-// the dispersive-cell kernel for the job's kinds: the gold update's own
-// instance when every dispersive material runs it
-template <typename T, int L>
-void launch_ade(const StepParams<T> &p, int blocks, cudaStream_t s, bool pdl) {
-  if (p.ade_kind == MK_GOLD) {
-    if (pdl) launch_pdl(e2d_ade<T, L, MK_GOLD>, blocks, 256, s, p);
-    else launch_side(e2d_ade<T, L, MK_GOLD>, blocks, 256, s, p);
-  } else {
-    if (pdl) launch_pdl(e2d_ade<T, L, -1>, blocks, 256, s, p);
-    else launch_side(e2d_ade<T, L, -1>, blocks, 256, s, p);
-  }
-}
-
 // The E half's side kernel when the job has dispersive cells: the edge
 // units' blocks, then the dispersive cells' blocks, in one launch beside the
 // core kernel (one branch of the step's graph instead of two)
@@ -629,7 +606,7 @@ __global__ void __launch_bounds__(256) e2d_edge_ade(const __grid_constant__ Step
 // kernels launch with the device's top priority
 template <typename T, int L, int V>
 int launch_e2d_v(const StepParams<T> &p, int part, cudaStream_t s, cudaEvent_t ev) {
-  const int units = part == K2D_CORE ? p.ncore : part == K2D_EDGE ? p.nedge + p.nade : p.nade;
+  const int units = part == K2D_CORE ? p.ncore : part == K2D_EDGE ? p.nedge + p.nade : 0;
   if (units <= 0) return 0;
   const int blocks = (units + 255) / 256;
   if (part == K2D_CORE) launch_core2_tiled<T, L, V>(p, true, s, ev);
@@ -638,8 +615,7 @@ int launch_e2d_v(const StepParams<T> &p, int part, cudaStream_t s, cudaEvent_t e
     if (p.ade_kind == MK_GOLD) launch_side(e2d_edge_ade<T, L, V, MK_GOLD>, b2, 256, s, p);
     else launch_side(e2d_edge_ade<T, L, V, -1>, b2, 256, s, p);
   }
-  else if (part == K2D_EDGE) launch_side(e2d_edge<T, L, V>, blocks, 256, s, p);
-  else launch_ade<T, L>(p, blocks, s, false);
+  else launch_side(e2d_edge<T, L, V>, blocks, 256, s, p);
   return 1;
 }
 template <typename T, int L, int V>
@@ -660,15 +636,6 @@ int launch_e2d(const StepParams<T> &p, int part, void *stream, void *prog_event)
   if (p.layout == 3)
     return p.vec == VW ? launch_e2d_v<T, 3, VW>(p, part, s, ev) : launch_e2d_v<T, 3, 1>(p, part, s, ev);
   return p.vec == VW ? launch_e2d_v<T, 2, VW>(p, part, s, ev) : launch_e2d_v<T, 2, 1>(p, part, s, ev);
-}
-
-template <typename T>
-int launch_e2d_ade_pdl(const StepParams<T> &p, void *stream) {
-  if (p.nade <= 0) return 0;
-  cudaStream_t s = (cudaStream_t)stream;
-  if (p.layout == 3) launch_ade<T, 3>(p, (p.nade + 255) / 256, s, true);
-  else launch_ade<T, 2>(p, (p.nade + 255) / 256, s, true);
-  return 1;
 }
 
 template <typename T>
@@ -783,7 +750,5 @@ template int launch_e2d<float>(const StepParams<float> &, int, void *, void *);
 template int launch_e2d<double>(const StepParams<double> &, int, void *, void *);
 template int launch_h2d<float>(const StepParams<float> &, int, void *, void *);
 template int launch_h2d<double>(const StepParams<double> &, int, void *, void *);
-template int launch_e2d_ade_pdl<float>(const StepParams<float> &, void *);
-template int launch_e2d_ade_pdl<double>(const StepParams<double> &, void *);
 
 }  // namespace fdtd

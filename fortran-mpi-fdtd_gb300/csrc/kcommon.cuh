@@ -30,6 +30,12 @@ __device__ __forceinline__ double lin2(double a, double b, double c, double d) {
   return __fma_rn(a, b, __dmul_rn(c, d));
 }
 
+// a*b + c, fused; a*b, rounded by itself
+__device__ __forceinline__ float fma1(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fma1(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float mul1(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul1(double a, double b) { return __dmul_rn(a, b); }
+
 // launch a step kernel with a programmatic dependency on the kernel before it
 // on the stream (the kernel starts with pdl_wait).  With `ev`, the launch also
 // records ev as a programmatic event that fires once every block has started:
@@ -454,16 +460,18 @@ __device__ __forceinline__ T *stage_ring(const StepParams<T> &p) {
   return p.d_half ? p.stage + (long long)(*p.d_half) * kStageSteps * p.stage_row : p.stage;
 }
 
-// Fused sampling: write the monitored components of cell (i,j,k) into this
-// step's stage row, and probe samples.  vals[c] = value of component c.
+// Fused sampling: write the monitored components of cell (i,j,k) into the stage
+// row of `slot` (unless `mons` is false), and probe samples.  vals[c] = value of
+// component c.
 template <typename T>
-__device__ __forceinline__ void gather_cell(const StepParams<T> &p, int n, int i, int j, int k, const T *vals) {
-  for (int q = 0; q < p.nmon; ++q) {
+__device__ __forceinline__ void gather_cell(const StepParams<T> &p, int n, int i, int j, int k, const T *vals, int slot,
+                                            bool mons = true) {
+  for (int q = 0; mons && q < p.nmon; ++q) {
     const Monitor &m = p.mon[q];
     if (i < m.lo[0] || i > m.hi[0] || j < m.lo[1] || j > m.hi[1] || k < m.lo[2] || k > m.hi[2]) continue;
     const int wx = m.hi[0] - m.lo[0] + 1, wy = m.hi[1] - m.lo[1] + 1;
     const long long idx = (long long)(i - m.lo[0]) + (long long)wx * ((j - m.lo[1]) + (long long)wy * (k - m.lo[2]));
-    T *row = stage_ring(p) + (long long)p.slot * p.stage_row + m.base;
+    T *row = stage_ring(p) + (long long)slot * p.stage_row + m.base;
     for (int u = 0; u < m.ncomp; ++u) row[(long long)u * m.ncell + idx] = pick6(vals, m.comps[u]);
   }
   for (int q = 0; q < p.nprobe; ++q) {

@@ -439,11 +439,11 @@ int fdtd_estimate_bytes(const fdtd_job *job, uint64_t *bytes);
  * (core) kernels; FDTD_KERNEL_EDGE: the 2D kernels for PML cells, the edges
  * of the main range and rows with sources, monitors or reference slabs (in
  * 3D with the fused step kernel: the general E and H kernels);
- * FDTD_KERNEL_ADE: the 2D dispersive-cell kernel of the fused step (the
- * split 2D step appends the dispersive cells' blocks to its E edge kernel,
- * timed as FDTD_KERNEL_EDGE); FDTD_KERNEL_STEP: the
- * fused step kernels (3D: E and H of the core box in one launch; 2D: E and
- * H of the whole grid, dispersive cells aside, in one launch). */
+ * FDTD_KERNEL_ADE: no launch of its own any more (the split 2D step appends
+ * the dispersive cells' blocks to its E edge kernel, timed as
+ * FDTD_KERNEL_EDGE); FDTD_KERNEL_STEP: the fused 3D step kernel (E and H of
+ * the core box in one launch) and the 2D block-step kernels (the whole grid,
+ * up to eight steps in one timed pair of launches). */
 enum { FDTD_KERNEL_E = 0, FDTD_KERNEL_H = 1, FDTD_KERNEL_DFT = 2, FDTD_KERNEL_LINE1D = 3,
        FDTD_KERNEL_EDGE = 4, FDTD_KERNEL_ADE = 5, FDTD_KERNEL_STEP = 6, FDTD_KERNEL_COUNT = 7 };
 int fdtd_profile(fdtd_job *job, int32_t enable);
@@ -452,11 +452,12 @@ int fdtd_kernel_time(fdtd_job *job, int32_t kind, int64_t *launches, double *ms)
  * (the default) lets commit time the candidates on the job's own grid and
  * keep the fastest (cached per kind of grid; environment FDTD_TUNE=0 skips
  * the timing); 1..3 pins a candidate: 2D 128 / 256 / 512 threads per block
- * (2D 4: the fused step kernel, which takes Ez, Hx and Hy of every cell
- * from step n to n+1 in one pass over two sets of field buffers used in
- * turn, for TMz FP32 jobs with nx a multiple of 4, no periodic axis and no
- * reference slabs, TFSF box or mean monitors; the job then holds a second
- * copy of its fields and of the stored PML part),
+ * (2D 4: the block-step kernel, which takes the whole grid up to eight steps
+ * on in one launch, over two sets of field buffers used in turn; the tuner
+ * offers it to FP32 jobs without reference slabs, TFSF box or mean monitors,
+ * and it can be pinned for TMz FP32 jobs with nx a multiple of 4 and no
+ * periodic axis among these; the job then holds a second copy of its fields,
+ * of the stored PML part and of its dispersive state),
  * 3D 4 / 8 / 16 rows of 32 x-vectors, one plane per thread; 3D also 4..6:
  * the same shapes with each thread walking 8 planes and keeping the
  * neighbour plane in registers.  FP32 with 4-cell vectors, where the core
