@@ -344,7 +344,7 @@ int kernel_flag(fdtd_job *J) {
   int h = 0;
   CK(cudaMemcpy(&h, J->d_err, sizeof h, cudaMemcpyDeviceToHost));
   if (!h) return FDTD_OK;
-  CK(cudaMemset(J->d_err, 0, sizeof h));
+  CK(cudaMemsetAsync(J->d_err, 0, sizeof h, J->stream));
   return set_err(FDTD_ECUDA, "a bounded wait in the TMA core kernel gave up");
 }
 
@@ -358,12 +358,17 @@ int alloc_state(fdtd_job *J, void **p, size_t bytes, int esz = 0) {
   return FDTD_OK;
 }
 
+// Host data go to the device on the job's stream: a plain cudaMemcpy from
+// pageable memory may return before its last bytes have landed, and the job's
+// streams, which do not wait for the legacy stream, could then run ahead of it
+// (seen on a busy GPU: a source table read before it was there).  The copy has
+// left the host buffer when the call returns.
 template <typename T>
 int upload_vec(fdtd_job *J, void **dst, const std::vector<double> &v) {
   std::vector<T> t(v.begin(), v.end());
   int rc = alloc_dev(J, dst, t.size() * sizeof(T));
   if (rc) return rc;
-  CK(cudaMemcpy(*dst, t.data(), t.size() * sizeof(T), cudaMemcpyHostToDevice));
+  CK(cudaMemcpyAsync(*dst, t.data(), t.size() * sizeof(T), cudaMemcpyHostToDevice, J->stream));
   J->h2d += t.size() * sizeof(T);
   return FDTD_OK;
 }
@@ -538,7 +543,7 @@ int split_2d(fdtd_job *J, const std::vector<uint8_t> &rf) {
   int rc;
   if (!edge.empty()) {
     if ((rc = alloc_dev(J, (void **)&J->d_edge, edge.size() * sizeof(int)))) return rc;
-    CK(cudaMemcpy(J->d_edge, edge.data(), edge.size() * sizeof(int), cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(J->d_edge, edge.data(), edge.size() * sizeof(int), cudaMemcpyHostToDevice, J->stream));
     J->h2d += edge.size() * sizeof(int);
   }
   return make_branches(J);
@@ -579,7 +584,7 @@ int split_3d(fdtd_job *J, const std::vector<uint8_t> &rf) {
   int rc;
   if (!edge.empty()) {
     if ((rc = alloc_dev(J, (void **)&J->d_edge, edge.size() * sizeof(int)))) return rc;
-    CK(cudaMemcpy(J->d_edge, edge.data(), edge.size() * sizeof(int), cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(J->d_edge, edge.data(), edge.size() * sizeof(int), cudaMemcpyHostToDevice, J->stream));
     J->h2d += edge.size() * sizeof(int);
   }
   return make_branches(J);
@@ -964,10 +969,10 @@ int commit_impl(fdtd_job *J) {
       }
   }
   if ((rc = alloc_dev(J, (void **)&J->d_mat, (size_t)N))) return rc;
-  CK(cudaMemcpy(J->d_mat, mat.data(), (size_t)N, cudaMemcpyHostToDevice));
+  CK(cudaMemcpyAsync(J->d_mat, mat.data(), (size_t)N, cudaMemcpyHostToDevice, J->stream));
   J->h2d += (uint64_t)N;
   if ((rc = alloc_dev(J, &J->d_mc, sizeof(MatCoef<T>) * kMaxMat))) return rc;
-  CK(cudaMemcpy(J->d_mc, mc.data(), sizeof(MatCoef<T>) * kMaxMat, cudaMemcpyHostToDevice));
+  CK(cudaMemcpyAsync(J->d_mc, mc.data(), sizeof(MatCoef<T>) * kMaxMat, cudaMemcpyHostToDevice, J->stream));
   J->h2d += sizeof(MatCoef<T>) * kMaxMat + sizeof(AdeCoef<T>) * ac.size();
   {
     std::vector<double> ca(kMaxMat, 0.0), cs(kMaxMat, 0.0);
@@ -978,7 +983,7 @@ int commit_impl(fdtd_job *J) {
     if ((rc = upload_vec<T>(J, &J->d_mcs, cs))) return rc;
   }
   if ((rc = alloc_dev(J, &J->d_ac, sizeof(AdeCoef<T>) * std::max<size_t>(1, ac.size())))) return rc;
-  if (!ac.empty()) CK(cudaMemcpy(J->d_ac, ac.data(), sizeof(AdeCoef<T>) * ac.size(), cudaMemcpyHostToDevice));
+  if (!ac.empty()) CK(cudaMemcpyAsync(J->d_ac, ac.data(), sizeof(AdeCoef<T>) * ac.size(), cudaMemcpyHostToDevice, J->stream));
   J->ac_host.assign((const char *)ac.data(), (const char *)ac.data() + sizeof(AdeCoef<T>) * ac.size());
   J->ade_kind = ac.empty() ? -1 : ac[0].kind;  // the device update all the dispersive materials share, or -1
   for (const AdeCoef<T> &a : ac)
@@ -1008,8 +1013,8 @@ int commit_impl(fdtd_job *J) {
   if ((rc = alloc_dev(J, (void **)&J->d_ade_cell, sizeof(int) * std::max(1, J->nade)))) return rc;
   if ((rc = alloc_dev(J, (void **)&J->d_ade_mat, std::max(1, J->nade)))) return rc;
   if (J->nade) {
-    CK(cudaMemcpy(J->d_ade_cell, ade_cell.data(), sizeof(int) * J->nade, cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(J->d_ade_mat, ade_mat.data(), J->nade, cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(J->d_ade_cell, ade_cell.data(), sizeof(int) * J->nade, cudaMemcpyHostToDevice, J->stream));
+    CK(cudaMemcpyAsync(J->d_ade_mat, ade_mat.data(), J->nade, cudaMemcpyHostToDevice, J->stream));
     J->h2d += (uint64_t)J->nade * (sizeof(int) + 1);
   }
   J->ade_nf = 0;
@@ -1171,7 +1176,7 @@ int commit_impl(fdtd_job *J) {
       for (int j = 0; j < ny; ++j)
         if (j < J->slab_rows || j >= ny - J->slab_rows) rf[j] |= ROW_SLAB;
     if ((rc = alloc_dev(J, (void **)&J->d_rowflag, (size_t)ny))) return rc;
-    CK(cudaMemcpy(J->d_rowflag, rf.data(), (size_t)ny, cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(J->d_rowflag, rf.data(), (size_t)ny, cudaMemcpyHostToDevice, J->stream));
     J->h2d += (uint64_t)ny;
     if ((rc = split_2d(J, rf))) return rc;
   } else if (J->dim == 3) {
@@ -1183,7 +1188,7 @@ int commit_impl(fdtd_job *J) {
           rf[(size_t)k * ny + j] |= ROW_SRC;
     }
     if ((rc = alloc_dev(J, (void **)&J->d_rowflag, rf.size()))) return rc;
-    CK(cudaMemcpy(J->d_rowflag, rf.data(), rf.size(), cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(J->d_rowflag, rf.data(), rf.size(), cudaMemcpyHostToDevice, J->stream));
     J->h2d += rf.size();
     if ((rc = split_3d(J, rf))) return rc;
   }
@@ -1205,7 +1210,7 @@ int commit_impl(fdtd_job *J) {
       }
     }
     if ((rc = alloc_dev(J, (void **)&J->d_uni, bits.size() * sizeof(uint32_t)))) return rc;
-    CK(cudaMemcpy(J->d_uni, bits.data(), bits.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(J->d_uni, bits.data(), bits.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, J->stream));
     J->h2d += bits.size() * sizeof(uint32_t);
     J->uni_words = words;
   }
@@ -1213,7 +1218,7 @@ int commit_impl(fdtd_job *J) {
   J->acc_total = acc;
   if (!omega.empty()) {
     if ((rc = alloc_dev(J, (void **)&J->d_omega, omega.size() * sizeof(double)))) return rc;
-    CK(cudaMemcpy(J->d_omega, omega.data(), omega.size() * sizeof(double), cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(J->d_omega, omega.data(), omega.size() * sizeof(double), cudaMemcpyHostToDevice, J->stream));
     // e^{i w s dt} for the slots of a DFT ring
     std::vector<double> rot(omega.size() * 2 * kStageSteps);
     for (size_t f = 0; f < omega.size(); ++f)
@@ -1223,7 +1228,7 @@ int commit_impl(fdtd_job *J) {
         rot[(f * kStageSteps + sl) * 2 + 1] = std::sin(ph);
       }
     if ((rc = alloc_dev(J, (void **)&J->d_rot, rot.size() * sizeof(double)))) return rc;
-    CK(cudaMemcpy(J->d_rot, rot.data(), rot.size() * sizeof(double), cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(J->d_rot, rot.data(), rot.size() * sizeof(double), cudaMemcpyHostToDevice, J->stream));
     J->h2d += rot.size() * sizeof(double);
     J->h2d += omega.size() * sizeof(double);
   }
@@ -1395,7 +1400,7 @@ int setup_block(fdtd_job *J) {
     *dst = nullptr;
     B.bytes[q] = bytes;
     if (const int e = alloc_dev(J, dst, bytes)) return e;
-    if (src) CK(cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice));
+    if (src) CK(cudaMemcpyAsync(*dst, src, bytes, cudaMemcpyHostToDevice, J->stream));
     J->h2d += src ? bytes : 0;
     return FDTD_OK;
   };
@@ -1721,7 +1726,7 @@ int ensure_srctab(fdtd_job *J, int n_max) {
     J->srctab_cap_steps = cap;
     J->dev_bytes += (uint64_t)cap * nsrc * sizeof(double);
     destroy_graph(J);  // the captured launches hold the old pointer
-    CK(cudaMemcpy(J->d_srctab, J->srctab.data(), (size_t)n_max * nsrc * sizeof(double), cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(J->d_srctab, J->srctab.data(), (size_t)n_max * nsrc * sizeof(double), cudaMemcpyHostToDevice, J->stream));
   } else {
     CK(cudaMemcpyAsync(J->d_srctab + (size_t)old_steps * nsrc, J->srctab.data() + (size_t)old_steps * nsrc,
                        (size_t)(n_max - old_steps) * nsrc * sizeof(double), cudaMemcpyHostToDevice, J->stream));
@@ -3299,14 +3304,14 @@ int fdtd_load_state(fdtd_job *J, const void *buf, uint64_t bytes) {
   if (n_probe_max > 0 && (rc = ensure_probe_cap(J, n_probe_max))) return rc;
   const char *o = pr + J->probes.size() * 2 * sizeof(int32_t);
   for (auto &s : J->state) {
-    CK(cudaMemcpy(s.p, o, s.bytes, cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(s.p, o, s.bytes, cudaMemcpyHostToDevice, J->stream));
     o += s.bytes;
   }
   for (size_t q = 0; q < J->probes.size(); ++q) {
     ProbeRec &P = J->probes[q];
     const size_t b = (size_t)caps[q] * P.ncomp * sizeof(double);
-    if (P.buf && P.cap > 0) CK(cudaMemset(P.buf, 0, (size_t)P.cap * P.ncomp * sizeof(double)));
-    if (b) CK(cudaMemcpy(P.buf, o, b, cudaMemcpyHostToDevice));
+    if (P.buf && P.cap > 0) CK(cudaMemsetAsync(P.buf, 0, (size_t)P.cap * P.ncomp * sizeof(double), J->stream));
+    if (b) CK(cudaMemcpyAsync(P.buf, o, b, cudaMemcpyHostToDevice, J->stream));
     o += b;
   }
   J->stage_fill = h.stage_fill;

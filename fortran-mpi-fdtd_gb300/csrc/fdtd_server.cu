@@ -173,7 +173,8 @@ void commit_worker(fdtd_server *S) {
 // rings up to chunk_steps.
 bool advance_packs(fdtd_server *S, std::unique_lock<std::mutex> &lk) {
   bool progressed = false;
-  for (Req *r : S->active)
+  const std::vector<Req *> now = S->active;  // the lock is let go of below: commits may add to the list
+  for (Req *r : now)
     if (r->key >= 0 && !r->in_pack && !r->inflight && r->n_steps - r->next_n + 1 >= fdtd::kStageSteps &&
         S->groups[r->key].members.size() < (size_t)fdtd::kMaxPack && !S->groups[r->key].inflight) {
       S->groups[r->key].members.push_back(r);
