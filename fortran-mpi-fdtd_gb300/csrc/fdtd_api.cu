@@ -179,6 +179,10 @@ struct fdtd_job {
   // 1D line slabs [line][side]
   void *d_lex[2][2] = {}, *d_lhz[2][2] = {}, *d_lc[2][2][4] = {};
   int ja = -1, jb = -1;
+  // the 1D block-step kernel: its second set of buffers and each cell's
+  // dispersive slot (null lineB[0]: the job runs the cluster kernel)
+  void *lineB[4] = {}, *lineB_lex[2][2] = {}, *lineB_lhz[2][2] = {};
+  int *d_line_slot = nullptr;
   // sampling
   std::vector<Monitor> mon_dev;
   long long stage_row = 0;
@@ -594,6 +598,7 @@ template <typename T>
 int tune_tiles(fdtd_job *J);
 int setup_tma(fdtd_job *J);
 int setup_fused(fdtd_job *J);
+int setup_line(fdtd_job *J);
 
 void free_fused(fdtd_job *J);
 size_t ade_bytes(const fdtd_job *J);
@@ -1244,6 +1249,7 @@ int commit_impl(fdtd_job *J) {
   CK(cudaStreamSynchronize(J->stream));
   if ((rc = setup_tma(J))) return rc;
   if ((rc = setup_fused(J))) return rc;
+  if ((rc = setup_line(J))) return rc;
   if ((rc = tune_tiles<T>(J))) return rc;
   if (J->fused_ok && J->tile != fused_tile(J)) free_fused(J);  // the tuner kept a split shape
   std::vector<int>().swap(J->ade_cell_host);
@@ -1306,6 +1312,42 @@ int setup_tma(fdtd_job *J) {
   int rc;
   if (!J->d_err && (rc = alloc_dev(J, (void **)&J->d_err, sizeof(int)))) return rc;
   J->tma_ok = true;
+  return FDTD_OK;
+}
+
+// The 1D block-step kernel takes lines whose slabs continue the main range, with
+// the total-field boundary clear of them and not in a dispersive cell.  (Others
+// stay with the cluster kernel.)
+int setup_line(fdtd_job *J) {
+  if (J->dim != 1) return FDTD_OK;
+  const int N = J->ny, mlo = J->g.main_lo[1], mhi = J->g.main_hi[1];
+  if (N < 64 || mlo < 1 || mhi > N - 2 || mlo > mhi) return FDTD_OK;
+  if (J->slab_on[0] != J->slab_on[1]) return FDTD_OK;
+  if (J->slab_on[0] && (mlo != J->ja + 1 || mhi != J->jb - 1)) return FDTD_OK;
+  if (J->has_tfsf) {
+    const int bd = J->tfsf.boundary;
+    if (bd - 1 <= mlo || bd >= mhi) return FDTD_OK;
+    for (int c : J->ade_cell_host) if (c == bd) return FDTD_OK;
+  }
+  int rc;
+  const size_t w = J->esz;
+  for (int q = 0; q < (J->has_tfsf ? 4 : 2); ++q)
+    if ((rc = alloc_dev(J, &J->lineB[q], N * w))) return rc;
+  if (J->slab_on[0])
+    for (int l = 0; l < (J->has_tfsf ? 2 : 1); ++l)
+      for (int s = 0; s < 2; ++s) {
+        const size_t bytes = (size_t)(J->pml.npml[1][0] + 2) * w;
+        if ((rc = alloc_dev(J, &J->lineB_lex[l][s], bytes))) return rc;
+        if ((rc = alloc_dev(J, &J->lineB_lhz[l][s], bytes))) return rc;
+      }
+  if (J->nade > 0) {
+    std::vector<int> slot((size_t)N, -1);
+    for (int q = 0; q < J->nade; ++q) slot[J->ade_cell_host[q]] = q;
+    if ((rc = alloc_dev(J, (void **)&J->d_line_slot, N * sizeof(int)))) return rc;
+    CK(cudaMemcpyAsync(J->d_line_slot, slot.data(), N * sizeof(int), cudaMemcpyHostToDevice, J->stream));
+    J->h2d += N * sizeof(int);
+    if ((rc = alloc_dev(J, &J->ade_b, ade_bytes(J)))) return rc;
+  }
   return FDTD_OK;
 }
 
@@ -1816,7 +1858,15 @@ int dft_fold(fdtd_job *J) {
     d.stage_row = J->stage_row;
     d.total_work_blocks = J->dft_blocks;
     // fold in rings of kStageSteps rows (the 1D stage holds many rings)
-    for (int r0 = 0; r0 < J->stage_fill; r0 += kStageSteps) {
+    const bool rings = J->dim == 1 && J->stage_fill > kStageSteps && dft_rings_fit(d);
+    if (rings) {
+      d.nslots = J->stage_fill;
+      d.n0 = J->stage_n0;
+      ev_record(J, FDTD_KERNEL_DFT, true);
+      J->launches += launch_dft_rings<T>(d, (const T *)J->d_stage, J->stream);
+      ev_record(J, FDTD_KERNEL_DFT, false);
+    }
+    for (int r0 = 0; !rings && r0 < J->stage_fill; r0 += kStageSteps) {
       d.nslots = std::min(kStageSteps, J->stage_fill - r0);
       d.n0 = J->stage_n0 + r0;
       ev_record(J, FDTD_KERNEL_DFT, true);
@@ -2329,6 +2379,73 @@ int replay_ring(fdtd_job *J, int n0) {
   return FDTD_OK;
 }
 
+// The steps of p through the 1D block-step kernel, an even number of launches, so
+// that the state ends in the canonical buffers.  The host computes the sources'
+// values of the next launches while the GPU runs.
+// A block holds 128 V cells, ks of them on each side as halo.  A launch costs
+// 3.6 us besides its steps (loading, storing), a step 0.2 us: FP32 takes 32
+// steps (0.31 us a step on the 4000-cell gold line; 0.42 with 16).  FP64: its
+// pipe's time of a block's cells bounds a step, so 16 steps and less halo (the
+// 13004-cell stack without samples 1.18 us; 1.31 with 32, 1.48 with 8).  One cell
+// per thread until there are three blocks per SM, then two (us per step with one
+// / two cells; FP32: 14000 cells 0.302 / 0.316, 30000 0.316 / 0.317, 100000
+// 0.541 / 0.360; FP64: 30000 0.951 / 1.049, 100000 2.32 / 1.41).
+template <typename T, typename F>
+int line_blocks(fdtd_job *J, LineParams<T> p, T *stage, F sources) {
+  const bool f64 = sizeof(T) == 8;
+  const int ks = f64 ? 16 : kLineSteps;
+  const int V = p.N <= 3 * (128 - 2 * ks) * J->num_sms ? 1 : 2;
+  LineBlock<T> b{};
+  b.slot = J->d_line_slot;
+  if (p.nade > 0) {
+    const AdeCoef<T> *ac = reinterpret_cast<const AdeCoef<T> *>(J->ac_host.data());
+    b.one_gold = p.nac == 1 && ac[0].kind == MK_GOLD;
+    b.gold = ac[0];
+  }
+  b.stage = stage;
+  b.stage_row = J->stage_row;
+  T *A[4] = {p.ex, p.hz, p.exi, p.hzi}, *B[4];
+  T *const ade[2] = {p.ade_state, (T *)J->ade_b};
+  LineParams<T> q[2] = {p, p};  // reading either set
+  for (int c = 0; c < 4; ++c) B[c] = (T *)J->lineB[c];
+  q[1].ex = B[0]; q[1].hz = B[1]; q[1].exi = B[2]; q[1].hzi = B[3];
+  q[1].ade_state = ade[1];
+  for (int l = 0; l < 2; ++l)
+    for (int s = 0; s < 2; ++s) {
+      q[1].pex[l][s] = (T *)J->lineB_lex[l][s];
+      q[1].phz[l][s] = (T *)J->lineB_lhz[l][s];
+    }
+  int left = (p.n_steps + ks - 1) / ks;
+  left += left & 1;
+  ev_record(J, FDTD_KERNEL_LINE1D, true);
+  constexpr int kPiece = 256;  // steps whose source values are computed at once
+  int have = 0;
+  for (int s0 = 0, from = 0; left > 0; --left, from ^= 1) {
+    b.s0 = s0;
+    b.ks = (p.n_steps - s0 + left - 1) / left;
+    if (s0 + b.ks > have) {
+      const int to = std::min(p.n_steps, std::max(s0 + b.ks, have + kPiece));
+      if (const int rc = sources(have, to)) return rc;
+      have = to;
+    }
+    b.own = 128 * V - 2 * b.ks;
+    const LineParams<T> &out = q[from ^ 1];
+    b.exo = out.ex; b.hzo = out.hz; b.exio = out.exi; b.hzio = out.hzi;
+    b.ade_out = ade[from ^ 1];
+    for (int l = 0; l < 2; ++l)
+      for (int s = 0; s < 2; ++s) {
+        b.pexo[l][s] = out.pex[l][s];
+        b.phzo[l][s] = out.phz[l][s];
+      }
+    const int ran = launch_line1d_block<T>(q[from], b, V, J->stream);
+    if (!ran) return set_err(FDTD_ECUDA, "1D block-step launch: %s", cudaGetErrorString(cudaGetLastError()));
+    J->launches += ran;
+    s0 += b.ks;
+  }
+  ev_record(J, FDTD_KERNEL_LINE1D, false);
+  return FDTD_OK;
+}
+
 // 1D: the persistent line kernel over a chunk of steps
 template <typename T>
 int line_run(fdtd_job *J, int n_first, int n_steps, int stages) {
@@ -2379,31 +2496,34 @@ int line_run(fdtd_job *J, int n_first, int n_steps, int stages) {
     d.amp = s.amp;
     ++p.nsrc;
   }
-  if (p.nsrc) {
-    std::vector<double> v((size_t)n_steps * p.nsrc);
-    for (int st = 0; st < n_steps; ++st) {
+  if (p.nsrc && (long long)n_steps * p.nsrc > J->srcval_cap) {
+    // the new buffer first: if it cannot be had, the old one stays
+    const long long cap = std::max<long long>((long long)n_steps * p.nsrc, 4096);
+    double *nb = nullptr;
+    cudaError_t e = pool_alloc(J, (void **)&nb, cap * sizeof(double));
+    if (e != cudaSuccess) return set_err(FDTD_ENOMEM, "source values: %s", cudaGetErrorString(e));
+    if (J->d_srcval) { pool_free(J, J->d_srcval); J->dev_bytes -= J->srcval_cap * sizeof(double); }
+    J->d_srcval = nb;
+    J->srcval_cap = cap;
+    J->dev_bytes += cap * sizeof(double);
+  }
+  // the sources' values of steps st0..st1-1 of the call, to the device
+  auto sources = [&](int st0, int st1) -> int {
+    if (!p.nsrc || st1 <= st0) return FDTD_OK;
+    std::vector<double> v((size_t)(st1 - st0) * p.nsrc);
+    for (int st = st0; st < st1; ++st) {
       const double t = (double)(n_first + st - 1) * J->g.dt;
       int q = 0;
       for (auto &s : J->srcs) {
         const double g = gauss_t(s, t);
-        v[(size_t)st * p.nsrc + q] = s.component == FDTD_EX_INC ? g : g * s.amp;
+        v[(size_t)(st - st0) * p.nsrc + q] = s.component == FDTD_EX_INC ? g : g * s.amp;
         ++q;
       }
     }
-    if ((long long)v.size() > J->srcval_cap) {
-      // the new buffer first: if it cannot be had, the old one stays
-      const long long cap = std::max<long long>((long long)v.size(), 4096);
-      double *nb = nullptr;
-      cudaError_t e = pool_alloc(J, (void **)&nb, cap * sizeof(double));
-      if (e != cudaSuccess) return set_err(FDTD_ENOMEM, "source values: %s", cudaGetErrorString(e));
-      if (J->d_srcval) { pool_free(J, J->d_srcval); J->dev_bytes -= J->srcval_cap * sizeof(double); }
-      J->d_srcval = nb;
-      J->srcval_cap = cap;
-      J->dev_bytes += cap * sizeof(double);
-    }
-    CK(cudaMemcpyAsync(J->d_srcval, v.data(), v.size() * sizeof(double), cudaMemcpyHostToDevice, J->stream));
-    CK(cudaStreamSynchronize(J->stream));  // v is a temporary
-  }
+    CK(cudaMemcpyAsync(J->d_srcval + (size_t)st0 * p.nsrc, v.data(), v.size() * sizeof(double), cudaMemcpyHostToDevice,
+                       J->stream));  // pageable: v has been read when the call returns
+    return FDTD_OK;
+  };
   p.srcval = J->d_srcval;
   p.nmon = (int)J->mon_dev.size();
   for (int q = 0; q < p.nmon; ++q) p.mon[q] = J->mon_dev[q];
@@ -2424,10 +2544,17 @@ int line_run(fdtd_job *J, int n_first, int n_steps, int stages) {
   p.n_steps = n_steps;
   p.stages = stages;
   T *stage = (T *)J->d_stage + (size_t)J->stage_fill * J->stage_row;
-  ev_record(J, FDTD_KERNEL_LINE1D, true);
-  launch_line1d_stage<T>(p, stage, J->stage_row, J->stream);
-  ev_record(J, FDTD_KERNEL_LINE1D, false);
-  J->launches++;
+  int rc;
+  if (J->lineB[0] && stages == (ST_E | ST_H | ST_SAMPLE) && n_steps > 1) {
+    rc = line_blocks<T>(J, p, stage, sources);
+  } else {
+    if ((rc = sources(0, n_steps))) return rc;
+    ev_record(J, FDTD_KERNEL_LINE1D, true);
+    launch_line1d_stage<T>(p, stage, J->stage_row, J->stream);
+    ev_record(J, FDTD_KERNEL_LINE1D, false);
+    J->launches++;
+  }
+  if (rc) return rc;
   CK(cudaGetLastError());
   return FDTD_OK;
 }
@@ -3436,6 +3563,8 @@ int fdtd_estimate_bytes(const fdtd_job *J, uint64_t *bytes) {
   // (at least 112 x 16 cells, 96 bytes with their flags)
   const bool block2 = J->dim == 2 && w == 4 && !J->has_tfbox && !(J->has_pml && J->pml.mode == FDTD_PML_REFERENCE);
   if (block2) b += 4 * N * w + ((uint64_t)nx / 112 + 1) * ((uint64_t)ny / 16 + 1) * 96;
+  if (J->dim == 1)  // the 1D block-step kernel's second set and slot map
+    b += (J->has_tfsf ? 4 : 2) * N * w + 4 * N + 8ull * (J->pml.npml[1][0] + 2) * w;
   if (J->has_tfsf) b += 2 * N * w;
   if (J->has_tfbox) b += 2ull * ny * w + 4 * w;
   // dispersive cells: each region's cells, bounded per sphere / box
@@ -3466,6 +3595,7 @@ int fdtd_estimate_bytes(const fdtd_job *J, uint64_t *bytes) {
   b += nade * ((uint64_t)nf * 3 * w + 5) + 32ull * nf * 3 * w;
   // and its dispersive cells: a second state, and in up to four tiles a list
   // entry and the scratch state
+  if (J->dim == 1) b += nade * (uint64_t)nf * 3 * w + 32ull * nf * 3 * w;
   if (block2) b += nade * ((uint64_t)nf * 3 * w + 4 * (8 + 2ull * nf * w)) + 32ull * nf * 3 * w;
   if (J->has_pml && J->pml.mode == FDTD_PML_SPLIT) {
     b += (uint64_t)(J->dim == 3 ? 6 : 1) * (w == 8 ? 2 : 1) * N * w;

@@ -373,6 +373,10 @@ struct DftParams {
   int total_work_blocks;
 };
 template <typename T> void launch_dft(const DftParams &d, const T *stage, void *stream);
+// every ring of a line's stage in one launch, for monitors of few samples
+// (dft_rings_fit); d.nslots: the rows of all of them.  Returns the launches.
+bool dft_rings_fit(const DftParams &d);
+template <typename T> int launch_dft_rings(DftParams d, const T *stage, void *stream);
 // load the DFT fold kernel on the current device now (cudaFuncGetAttributes)
 // rather than at its first launch; 0 on success
 template <typename T> int preload_dft();
@@ -416,6 +420,24 @@ struct LineParams {
   int n_first, n_steps;
   int stages;              // bit0: E half, bit1: H half, bit2: sample
 };
+// a block of steps of the line per launch (k1b.cu): from p's buffers to the other
+// set, b's
+constexpr int kLineSteps = 32;
+template <typename T>
+struct LineBlock {
+  T *exo, *hzo, *exio, *hzio;
+  T *pexo[2][2], *phzo[2][2];  // slab arrays [line][side]
+  T *ade_out;
+  const int *slot;             // per cell: its dispersive slot
+  int one_gold;                // every dispersive cell is of one gold material, `gold`
+  AdeCoef<T> gold;
+  T *stage;                    // row of the first step of p
+  long long stage_row;
+  int s0, ks, own;             // first step of this launch (from p.n_first), its steps, cells per block
+};
+// V: cells per thread (1 or 2; a block holds 128 V cells, own + 2 ks of them);
+// returns the kernels launched
+template <typename T> int launch_line1d_block(const LineParams<T> &p, const LineBlock<T> &b, int V, void *stream);
 template <typename T> void launch_line1d_stage(const LineParams<T> &p, T *stage, long long stage_row, void *stream);
 
 // Records a message for fdtd_last_error and returns `code`.

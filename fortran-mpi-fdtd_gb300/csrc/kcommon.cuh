@@ -374,6 +374,143 @@ __device__ __forceinline__ T ade_update_state(T *st, int stride, int slot, int c
   return e;
 }
 
+// ade_update_state with the state as [field][NC][slot], for the kernels that take
+// several steps per launch.  The roundings of its sums of products are written
+// out, as the compiler chose them in the one-step kernels: left to it here, other
+// choices would part the two paths in the last bit.
+template <typename T, int KIND, int NC>
+__device__ __forceinline__ T ade_update_fixed(T *st, int stride, int slot, int comp, const AdeCoef<T> &a,
+                                               const AdeCoef<T> *am, T inc, T eold) {
+  const int kind = KIND >= 0 ? KIND : a.kind;
+  T *q_ = st + (0 * NC + comp) * (long long)stride + slot;
+  T *s_ = st + (1 * NC + comp) * (long long)stride + slot;
+  T *f2 = st + (2 * NC + comp) * (long long)stride + slot;
+  T *f3 = st + (3 * NC + comp) * (long long)stride + slot;
+  if (kind == MK_LORENTZ) {
+    if (comp == a.normal) return eold + inc;  // sheet: the normal component is vacuum
+    T pl[kMaxPoles], vl[kMaxPoles];
+    T sv = T(0);
+#pragma unroll
+    for (int l = 0; l < kMaxPoles; ++l) {
+      if (l < a.npoles) {
+        pl[l] = st[(2 * l * NC + comp) * (long long)stride + slot];
+        vl[l] = st[((2 * l + 1) * NC + comp) * (long long)stride + slot];
+        sv += vl[l];
+      }
+    }
+    const int nlf = 2 * a.npoles;  // the Kerr term's Q and g follow the poles
+    if (a.zx) {
+      // SLG_LJp's Ez line subtracts the x current of the previous step
+      // (3D/grapheneLorentzJp_mod.f90:68): the x update leaves its sum in
+      // field nlf+2 (component slot 0) for the z update of the same cell
+      T *xs = st + ((nlf + 2) * NC) * (long long)stride + slot;
+      if (comp == 0) *xs = sv;
+      else if (comp == 2) sv = *xs;
+    }
+    const T e = eold + a.ga * (inc - sv);
+    T *qk = st + (nlf * NC + comp) * (long long)stride + slot, *gk = st + ((nlf + 1) * NC + comp) * (long long)stride + slot;
+    const T qv = a.nl ? *qk : T(0);
+#pragma unroll
+    for (int l = 0; l < kMaxPoles; ++l) {
+      if (l < a.npoles) {
+        T drive;
+        if (l == 0) {
+          drive = mul1(a.le[l], e);
+          if (a.nl) drive = fma1(a.lk, qv * e, drive);
+          drive = fma1(-a.ls[l], pl[l], drive);
+        } else {
+          drive = lin2(a.le[l], e, -a.ls[l], pl[l]);
+        }
+        const T nv = vl[l] + fma1(-a.lv[l], vl[l], drive);
+        st[((2 * l + 1) * NC + comp) * (long long)stride + slot] = nv;
+        st[(2 * l * NC + comp) * (long long)stride + slot] = pl[l] + nv;
+      }
+    }
+    if (a.nl) {
+      const T es = a.escale * e;
+      const T g = *gk;
+      const T ng = g + lin2(a.lqs, fma1(es, es, -qv), -a.lqv, g);
+      *gk = ng;
+      *qk = qv + ng;
+    }
+    return e;
+  }
+  T Q = *q_ + inc;
+  T S = *s_;
+  if (kind == MK_GOLD) {
+    T *f4 = st + (4 * NC + comp) * (long long)stride + slot;
+    T *f5 = st + (5 * NC + comp) * (long long)stride + slot;
+    const T g1r = *f2, g1i = *f3, g2r = *f4, g2i = *f5;
+    // gb*g = g + (gb-1)*g
+    const T p1r = g1r + lin2(a.dr[0], g1r, -a.di[0], g1i), p2r = g2r + lin2(a.dr[1], g2r, -a.di[1], g2i);
+    // (the half-step kernel of all-gold jobs rounds the second component's its own way)
+    const bool own = KIND == MK_GOLD && comp != 0;
+    const T p1i = g1i + (own ? lin2(a.dr[0], g1i, a.di[0], g1r) : lin2(a.di[0], g1r, a.dr[0], g1i));
+    const T p2i = g2i + (own ? lin2(a.dr[1], g2i, a.di[1], g2r) : lin2(a.di[1], g2r, a.dr[1], g2i));
+    const T nre = (fma1(a.ha, S, Q) + p1r) + p2r;
+    const T nim = p1i + p2i;
+    const T e = lin2(nre, a.wr, -nim, a.wi);
+    *q_ = fma1(-a.hb, e, Q);
+    *s_ = S + lin2(a.hb, e, -a.dha, S);
+    *f2 = fma1(a.gcr[0], e, p1r);
+    *f3 = fma1(a.gci[0], e, p1i);
+    *f4 = fma1(a.gcr[1], e, p2r);
+    *f5 = fma1(a.gci[1], e, p2i);
+    return e;
+  }
+  if (kind == MK_GRAPHENE_CP) {
+    // the reference's Graphene: Re[(Q + ha S + sum_p gb_p g_p) / (ga + S_R)].
+    // Its coefficients are read through am, not the caller's copy a: a copy
+    // of every kind's fields would stay in registers across the components.
+    if (comp == a.normal) return eold + inc;  // the normal component is vacuum (E = D)
+    const long long cs = NC * (long long)stride;
+    T *g0 = st + (2 * NC + comp) * (long long)stride + slot;  // g_p: fields 2+2p (re), 3+2p (im)
+    const T ha = am->ha, hb = am->hb, dha = am->dha;
+    T nre = fma1(ha, S, Q), nim = T(0);
+#pragma unroll 1  // unrolled, the loads of all four points would stay live together
+    for (int q = 0; q < kMaxCp; ++q) {
+      const T gr = g0[2 * q * cs], gi = g0[(2 * q + 1) * cs];
+      const T dr = am->dr[q], di = am->di[q];
+      nre = nre + (gr + lin2(dr, gr, -di, gi));
+      nim = nim + (gi + lin2(dr, gi, di, gr));
+    }
+    T *srp = st + (10 * NC + comp) * (long long)stride + slot, *vp = st + (11 * NC + comp) * (long long)stride + slot;
+    const T sr = *srp, v = *vp;
+    const T gai = am->gai, dre = am->gar + sr;
+    const T e = lin2(nim, gai, nre, dre) / lin2(gai, gai, dre, dre);
+    const T nv = fma1(am->r0, e * e, lin2(am->rv, v, am->rs, sr));
+    *vp = nv;
+    *srp = sr + nv;
+    *q_ = Q - mul1(hb, e);
+    *s_ = S + lin2(-dha, S, hb, e);
+    // g_p = gb_p g_p + gc_p E, with gb_p g_p recomputed from the state (the
+    // same operations as above, so the same values) rather than kept live
+#pragma unroll 1
+    for (int q = 0; q < kMaxCp; ++q) {
+      const T gr = g0[2 * q * cs], gi = g0[(2 * q + 1) * cs];
+      const T dr = am->dr[q], di = am->di[q];
+      g0[2 * q * cs] = fma1(am->gcr[q], e, gr + lin2(dr, gr, -di, gi));
+      g0[(2 * q + 1) * cs] = fma1(am->gci[q], e, gi + lin2(dr, gi, di, gr));
+    }
+    return e;
+  }
+  // graphene
+  if (comp == a.normal) {  // out-of-plane component: vacuum, E = D
+    *q_ = Q;
+    return eold + inc;
+  }
+  const T sr = *f2, v = *f3;
+  const T num = fma1(T(2) * a.kerr, eold * eold * eold, fma1(a.ha, S, Q));
+  const T den = fma1(T(3) * a.kerr, eold * eold, a.ga + sr);
+  const T e = num / den;
+  const T nv = fma1(a.r0, e * e, lin2(a.rv, v, a.rs, sr));
+  *f3 = nv;
+  *f2 = sr + nv;
+  *q_ = fma1(-a.hb, e, Q);
+  *s_ = S + lin2(a.hb, e, -a.dha, S);
+  return e;
+}
+
 // store V values, skipping cells whose E belongs to an ADE thread
 template <typename T, int V>
 __device__ __forceinline__ void st_guard3(T *a, const T (&v)[V], const uint8_t (&id)[V]) {
