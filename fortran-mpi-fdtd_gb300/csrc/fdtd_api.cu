@@ -241,6 +241,13 @@ struct fdtd_job {
     void *scratch = nullptr;
     size_t bytes[5] = {};  // of the five buffers
   } blk;
+  // the 3D block-step kernel: its tiles and tables, and the second sets of the
+  // stored split-PML parts
+  bool block3_ok = false;
+  bool lean = false;  // leave out every kernel that needs second sets of buffers
+  Block3 b3{};
+  void *spb3[6] = {};
+  size_t b3_bytes[6] = {};  // of the flags, slot map, first step's dispersive state, its sampled rows, order, segments
   std::vector<int> ade_cell_host;      // during commit: the dispersive cells and their ids
   std::vector<uint8_t> ade_mat_host;
   FusedMaps fmaps[2]{};
@@ -266,6 +273,7 @@ struct fdtd_job {
   int vec = 1, cv0 = 0, cw = 0, cy0 = 0, ncore = 0, nedge = 0;
   int ch = 0, cz0 = 0, cd = 0;  // 3D: core box rows and planes
   int tile_req = 0, tile = 1;    // core block shape: requested (0: tune) and used
+  int split_tile = 1;            // of the split kernels beside the 3D block-step kernel
   int *d_edge = nullptr;
   cudaStream_t side[2] = {};
   cudaEvent_t ev_fork = nullptr, ev_join[2] = {};
@@ -604,6 +612,8 @@ void free_fused(fdtd_job *J);
 size_t ade_bytes(const fdtd_job *J);
 // the tile (0-based) that selects the fused step kernel
 int fused_tile(const fdtd_job *J) { return J->dim == 3 ? 8 : 3; }
+constexpr int kBlock3Tile = 9;
+void free_block3(fdtd_job *J);
 
 // The TFSF box: faces, and the cells its face terms touch (the box widened by
 // one cell across each face) inside the grid, the main range and the PML's
@@ -1251,7 +1261,8 @@ int commit_impl(fdtd_job *J) {
   if ((rc = setup_fused(J))) return rc;
   if ((rc = setup_line(J))) return rc;
   if ((rc = tune_tiles<T>(J))) return rc;
-  if (J->fused_ok && J->tile != fused_tile(J)) free_fused(J);  // the tuner kept a split shape
+  if (J->block3_ok && J->tile != kBlock3Tile) free_block3(J);  // the tuner kept another shape
+  if (J->fused_ok && J->tile != fused_tile(J) && !J->block3_ok) free_fused(J);
   std::vector<int>().swap(J->ade_cell_host);
   std::vector<uint8_t>().swap(J->ade_mat_host);
   if ((rc = kernel_flag(J))) return rc;
@@ -1329,6 +1340,7 @@ int setup_line(fdtd_job *J) {
     if (bd - 1 <= mlo || bd >= mhi) return FDTD_OK;
     for (int c : J->ade_cell_host) if (c == bd) return FDTD_OK;
   }
+  if (J->lean) return FDTD_OK;
   int rc;
   const size_t w = J->esz;
   for (int q = 0; q < (J->has_tfsf ? 4 : 2); ++q)
@@ -1365,6 +1377,23 @@ void free_fused(fdtd_job *J) {
   for (int q = 0; q < 5; ++q) free_dev(J, tab[q], B.bytes[q]);
   B = fdtd_job::BlockTables{};
   J->fused_ok = false;
+}
+
+// the 3D block-step kernel's tables and second sets; the fields' second set
+// stays for the fused kernel
+void free_block3(fdtd_job *J) {
+  const size_t bytes = (size_t)J->ncell * J->esz;
+  for (int q = 0; q < 6; ++q) { free_dev(J, J->spb3[q], bytes); J->spb3[q] = nullptr; }
+  if (J->dim == 3) {
+    free_dev(J, J->ade_b, ade_bytes(J));
+    J->ade_b = nullptr;
+  }
+  void *const tab[6] = {(void *)J->b3.flags, (void *)J->b3.slot, J->b3.ade_mid, J->b3.first, (void *)J->b3.order, (void *)J->b3.seg};
+  for (int q = 0; q < 6; ++q) free_dev(J, tab[q], J->b3_bytes[q]);
+  J->b3 = Block3{};
+  J->block3_ok = false;
+  if (!J->fused_ok)
+    for (int c = 0; c < 6; ++c) { free_dev(J, J->Fb[c], bytes); J->Fb[c] = nullptr; }
 }
 
 // bytes of the dispersive state
@@ -1555,12 +1584,8 @@ void block_plan(const fdtd_job *J, BlockPlan &pl) {
 // update fields in place).  Its second set of field buffers is allocated
 // here, before the tuner times the kernel; commit gives it back if the tuner
 // keeps another shape.  Environment FDTD_NO_FUSED leaves the kernels out.
-int setup_fused(fdtd_job *J) {
-  J->fused_ok = false;
-  if (getenv("FDTD_NO_FUSED") || J->ncore <= 0) return FDTD_OK;
-  if (J->tile_req > 0 && J->tile_req != fused_tile(J) + 1) return FDTD_OK;  // another shape is pinned
-  if (J->dim == 2) return setup_block(J);
-  if (J->dim != 3 || !J->tma_ok || !J->tma.h_ok || J->slab_rows > 0 || J->has_tfbox) return FDTD_OK;
+int setup_fused3(fdtd_job *J) {
+  if (!J->tma_ok || !J->tma.h_ok) return FDTD_OK;
   PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
   if (!enc) return FDTD_OK;
   int rc;
@@ -1586,6 +1611,132 @@ int setup_fused(fdtd_job *J) {
   }
   J->fused_ok = true;
   return FDTD_OK;
+}
+
+template <typename T>
+void fill_common(fdtd_job *J, StepParams<T> &p);
+
+// The 3D block-step kernel takes any FP32 grid of even row length without
+// reference slabs or a TFSF box (those update fields in place), and materials
+// whose z update does not read the x update's current.
+int setup_block3(fdtd_job *J) {
+  if (J->esz != 4 || J->vec != 4 || J->nz < 2 || (unsigned long long)J->ncell >= 1ull << 30) return FDTD_OK;
+  const AdeCoef<float> *ac = reinterpret_cast<const AdeCoef<float> *>(J->ac_host.data());
+  for (size_t q = 0; q < J->ac_host.size() / sizeof(AdeCoef<float>); ++q)
+    if (ac[q].zx) return FDTD_OK;
+  int rc;
+  Block3 &b = J->b3;
+  block3_tiles(b, J->nx, J->ny, J->nz, J->num_sms);
+  const size_t bytes = (size_t)J->ncell * 4;
+  for (int c = 0; c < 6; ++c)
+    if (!J->Fb[c] && (rc = alloc_dev(J, &J->Fb[c], bytes))) return rc;
+  for (int q = 0; q < 6; ++q)
+    if (J->d_sp[q] && !J->spb3[q] && (rc = alloc_dev(J, &J->spb3[q], bytes))) return rc;
+  const size_t rows = (size_t)J->ny * J->nz * b.ntx;
+  J->b3_bytes[0] = rows;
+  if ((rc = alloc_dev(J, (void **)&b.flags, rows))) return rc;
+  {
+    StepParams<float> p;
+    fill_common<float>(J, p);
+    launch_row_flags3(p, b, (uint8_t *)b.flags, J->stream);
+    CK(cudaGetLastError());
+  }
+  std::vector<uint8_t> fl(rows);
+  CK(cudaMemcpyAsync(fl.data(), b.flags, rows, cudaMemcpyDeviceToHost, J->stream));
+  CK(cudaStreamSynchronize(J->stream));
+  // tiles with the most rows that are not plain first, so that no long one starts last
+  const int nt = b.ntx * b.nty * b.ntz;
+  std::vector<int> order((size_t)nt);
+  std::vector<long long> weight((size_t)nt, 0);
+  std::vector<char> ade((size_t)nt, 0);
+  for (int k = 0; k < J->nz; ++k)
+    for (int j = 0; j < J->ny; ++j)
+      for (int tx = 0; tx < b.ntx; ++tx) {
+        const uint8_t f = fl[((size_t)k * J->ny + j) * b.ntx + tx];
+        weight[((size_t)(k / b.oz) * b.nty + j / b.oy) * b.ntx + tx] += f & 4 ? 4 : f & 0x11 ? 1 : 0;
+        if (f & 64)  // in every tile whose halo reaches the row
+          tiles_of(k, J->nz, J->g.periodic[2], b.oz, 2, b.oz + 4, [&](int tz, int, bool) {
+            tiles_of(j, J->ny, J->g.periodic[1], b.oy, 1, b.oy + 3, [&](int ty, int, bool) { ade[((size_t)tz * b.nty + ty) * b.ntx + tx] = 1; });
+          });
+      }
+  for (int t = 0; t < nt; ++t) order[t] = t;
+  for (char c : ade) b.nade += c;
+  std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
+    return ade[x] != ade[y] ? ade[x] > ade[y] : weight[x] / 64 > weight[y] / 64;
+  });
+  J->b3_bytes[4] = (size_t)nt * sizeof(int);
+  if ((rc = alloc_dev(J, (void **)&b.order, J->b3_bytes[4]))) return rc;
+  CK(cudaMemcpyAsync((void *)b.order, order.data(), J->b3_bytes[4], cudaMemcpyHostToDevice, J->stream));
+  CK(cudaStreamSynchronize(J->stream));
+  J->h2d += J->b3_bytes[4];
+  if (J->nade > 0) {
+    b.one_gold = J->ac_host.size() == sizeof(AdeCoef<float>) && ac[0].kind == MK_GOLD;
+    int hi[3] = {0, 0, 0};
+    for (int a = 0; a < 3; ++a) b.alo[a] = INT32_MAX;
+    for (int c : J->ade_cell_host) {
+      const int x[3] = {c % J->nx, c / J->nx % J->ny, c / (J->nx * J->ny)};
+      for (int a = 0; a < 3; ++a) {
+        b.alo[a] = std::min(b.alo[a], x[a]);
+        hi[a] = std::max(hi[a], x[a]);
+      }
+    }
+    for (int a = 0; a < 3; ++a) b.an[a] = hi[a] - b.alo[a] + 1;
+    std::vector<int> slot((size_t)b.an[0] * b.an[1] * b.an[2], 0);
+    for (int q = 0; q < J->nade; ++q) {
+      const int c = J->ade_cell_host[q];
+      slot[((size_t)(c / (J->nx * J->ny) - b.alo[2]) * b.an[1] + (c / J->nx % J->ny - b.alo[1])) * b.an[0] + (c % J->nx - b.alo[0])] = q;
+    }
+    J->b3_bytes[1] = slot.size() * sizeof(int);
+    if ((rc = alloc_dev(J, (void **)&b.slot, J->b3_bytes[1]))) return rc;
+    CK(cudaMemcpyAsync((void *)b.slot, slot.data(), J->b3_bytes[1], cudaMemcpyHostToDevice, J->stream));
+    J->h2d += J->b3_bytes[1];
+    J->b3_bytes[2] = ade_bytes(J);
+    if ((rc = alloc_dev(J, (void **)&b.ade_mid, J->b3_bytes[2]))) return rc;
+    if (!J->ade_b && (rc = alloc_dev(J, &J->ade_b, ade_bytes(J)))) return rc;
+    CK(cudaStreamSynchronize(J->stream));
+  }
+  // the rows with samples, numbered
+  std::vector<int> seg(rows, 0);
+  int nseg = 0;
+  for (size_t r = 0; r < rows; ++r)
+    if (fl[r] & ROW_SAMPLE) seg[r] = nseg++;
+  if (nseg > 0) {
+    J->b3_bytes[3] = (size_t)nseg * 6 * b.ox * sizeof(float);
+    if ((rc = alloc_dev(J, (void **)&b.first, J->b3_bytes[3]))) return rc;
+    J->b3_bytes[5] = rows * sizeof(int);
+    if ((rc = alloc_dev(J, (void **)&b.seg, J->b3_bytes[5]))) return rc;
+    CK(cudaMemcpyAsync((void *)b.seg, seg.data(), J->b3_bytes[5], cudaMemcpyHostToDevice, J->stream));
+    J->h2d += J->b3_bytes[5];
+  }
+  CK(cudaStreamSynchronize(J->stream));
+  J->block3_ok = true;
+  return FDTD_OK;
+}
+
+// The step kernels that need second sets of buffers.  The block-step kernels are
+// left out where the device has no room for those: the split kernels need none.
+int setup_fused(fdtd_job *J) {
+  J->fused_ok = J->block3_ok = false;
+  if (getenv("FDTD_NO_FUSED") || J->ncore <= 0) return FDTD_OK;
+  if (J->tile_req > 0 && J->tile_req != fused_tile(J) + 1) return FDTD_OK;  // another shape is pinned
+  if (J->lean && J->tile_req == 0) return FDTD_OK;
+  if (J->dim == 2) {
+    const int rc = setup_block(J);
+    // TMz jobs of 4-cell rows have always had a second set and report its want
+    if (rc != FDTD_ENOMEM || (J->g.layout == FDTD_LAYOUT_2D_TM && J->vec == 4)) return rc;
+    cudaGetLastError();
+    free_fused(J);
+    return FDTD_OK;
+  }
+  if (J->dim != 3 || J->slab_rows > 0 || J->has_tfbox) return FDTD_OK;
+  int rc = setup_fused3(J);
+  if (rc || J->tile_req > 0) return rc;
+  if ((rc = setup_block3(J)) == FDTD_ENOMEM) {
+    cudaGetLastError();
+    free_block3(J);
+    rc = FDTD_OK;
+  }
+  return rc;
 }
 
 template <typename T>
@@ -1660,7 +1811,7 @@ void fill_common(fdtd_job *J, StepParams<T> &p) {
     p.vec = J->vec;
     p.cv0 = J->cv0; p.cw = J->cw; p.cy0 = J->cy0; p.ch = J->ch; p.cz0 = J->cz0; p.cd = J->cd;
     p.ncore = J->ncore;
-    p.tile = J->tile;
+    p.tile = J->tile == kBlock3Tile ? J->split_tile : J->tile;
   }
   if (J->has_tfbox) {
     p.tf_on = 1;
@@ -1967,11 +2118,23 @@ void block_buffers(const fdtd_job *J, StepParams<float> &p, BlockPlan &pl, int f
   }
   p.ex = A[0]; p.ey = A[1]; p.ez = A[2]; p.hx = A[3]; p.hy = A[4]; p.hz = A[5];
   p.exo = B[0]; p.eyo = B[1]; p.ezo = B[2]; p.hxo = B[3]; p.hyo = B[4]; p.hzo = B[5];
-  p.sp[0] = (float *)(from ? J->spb : J->d_sp[0]);
+  if (J->dim == 2) p.sp[0] = (float *)(from ? J->spb : J->d_sp[0]);
   p.spo = (float *)(from ? J->d_sp[0] : J->spb);
   p.ade_state = (float *)(from ? J->ade_b : J->d_ade_state);
   pl.ade_out = (float *)(from ? J->d_ade_state : J->ade_b);
   p.pp = 1;
+}
+
+// steps of the 3D block-step kernel: from set `from` to the other
+void block3_buffers(const fdtd_job *J, StepParams<float> &p, Block3 &b, int from) {
+  BlockPlan pl{};
+  block_buffers(J, p, pl, from);
+  b = J->b3;
+  b.ade_out = pl.ade_out;
+  for (int q = 0; q < 6; ++q) {
+    p.sp[q] = (float *)(from ? J->spb3[q] : J->d_sp[q]);
+    b.spo[q] = (float *)(from ? J->d_sp[q] : J->spb3[q]);
+  }
 }
 
 // The tiles of a block-step launch: general and plain ones write different
@@ -1989,6 +2152,23 @@ int launch_blocks(fdtd_job *J, const StepParams<float> &p, const BlockPlan &pl) 
   n += launch_step2d_block(p, pl, false, J->side[0]);
   if (!ok(cudaEventRecord(J->ev_join[0], J->side[0])) || !ok(cudaStreamWaitEvent(J->stream, J->ev_join[0], 0))) return -1;
   return n;
+}
+
+// The same in 3D: the tiles with dispersive cells beside the others, which run
+// without that code and its registers.
+int launch_blocks3(fdtd_job *J, const StepParams<float> &p, const Block3 &b, int k) {
+  const bool both = b.nade > 0 && b.nade < b.ntx * b.nty * b.ntz && !J->prof;
+  cudaStream_t side = both ? J->side[0] : J->stream;
+  cudaError_t e = cudaSuccess;
+  if (both && (e = cudaEventRecord(J->ev_fork, J->stream)) == cudaSuccess) e = cudaStreamWaitEvent(side, J->ev_fork, 0);
+  const int n0 = e == cudaSuccess ? launch_step3d_block(p, b, k, true, J->stream) : -1;
+  const int n1 = n0 >= 0 ? launch_step3d_block(p, b, k, false, side) : -1;
+  if (both && n1 >= 0 && (e = cudaEventRecord(J->ev_join[0], side)) == cudaSuccess) e = cudaStreamWaitEvent(J->stream, J->ev_join[0], 0);
+  if (n1 < 0 || e != cudaSuccess) {
+    set_err(FDTD_ECUDA, "3D block-step launch: %s", cudaGetErrorString(e != cudaSuccess ? e : cudaGetLastError()));
+    return -1;
+  }
+  return n0 + n1;
 }
 
 template <typename T>
@@ -2012,6 +2192,10 @@ int tune_tiles(fdtd_job *J) {
     J->tile = 1;
     return FDTD_OK;
   }
+  if (off && off[0] == 'b' && J->block3_ok) {  // "block": the 3D block-step kernel where it is offered
+    J->tile = kBlock3Tile;
+    return FDTD_OK;
+  }
   int lg = 0;
   for (long long c = J->ncore; c > 1; c >>= 1) ++lg;
   // which TMA-staged kernels the grid can take, and the share of dispersive
@@ -2020,12 +2204,14 @@ int tune_tiles(fdtd_job *J) {
   for (long long c = J->nade; lade < 15 && c < J->ncore; c *= 2, ++lade)
     if (c == 0) { lade = 15; break; }
   const long long key = ((((((long long)J->dim * 8 + J->g.layout) * 4 + J->g.precision) * 8 + J->vec) * 64 + lg) * 16 + lade) * 8 +
-                        (J->fused_ok ? 4 : 0) + (J->tma_ok ? 2 : 0) + (J->tma_ok && J->tma.h_ok ? 1 : 0);
+                        (J->fused_ok ? 4 : 0) + (J->tma_ok ? 2 : 0) + (J->tma_ok && J->tma.h_ok ? 1 : 0) +
+                        (J->block3_ok ? 1ll << 40 : 0);
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     auto it = g_tune.find(key);
     if (it != g_tune.end()) {
-      J->tile = it->second;
+      J->tile = it->second & 255;
+      J->split_tile = it->second >> 8;
       return FDTD_OK;
     }
   }
@@ -2035,7 +2221,7 @@ int tune_tiles(fdtd_job *J) {
   cudaEvent_t a = nullptr, b = nullptr;
   CK(cudaEventCreate(&a));
   CK(cudaEventCreate(&b));
-  float best = 3.0e38f;
+  float best = 3.0e38f, best_split = 3.0e38f;
   int choice = 1;
   // 3D: also the z-marching kernels and, where set up, the TMA-staged cores
   // and the fused step kernel (one launch in place of an E and an H core).
@@ -2043,23 +2229,47 @@ int tune_tiles(fdtd_job *J) {
   // step the edge and dispersive-cell kernels run beside the cores, and
   // their work is a small part of a grid large enough for the fused kernel)
   const int nshapes = J->dim == 3 ? (J->fused_ok ? 9 : J->tma_ok ? (J->tma.h_ok ? 8 : 7) : 6) : J->fused_ok ? 4 : 3;
-  // 2D: the block-step kernel takes whole steps, so it is timed against the
-  // whole split step of the best core shape: cores, edge and dispersive cells
+  // The block-step kernels take whole steps, so they are timed against the whole
+  // step of the best other shape: cores, edge and dispersive cells
   BlockPlan pl{};
   if (J->dim == 2 && J->fused_ok) block_plan(J, pl);
   auto split_step = [&] {
     const bool parts[3] = {true, true, false};
     p.roles = ROLE_MAIN | ROLE_PML | ROLE_ADE;
     p.tile = choice;
+    if constexpr (sizeof(T) == 4) {
+      if (J->dim == 3 && choice == fused_tile(J)) {
+        StepParams<float> q = p;
+        for (int u = 0; u < 3; ++u) {
+          float **const e[3] = {&q.exo, &q.eyo, &q.ezo}, **const h[3] = {&q.hxo, &q.hyo, &q.hzo};
+          *e[u] = (float *)J->Fb[u];
+          *h[u] = (float *)J->Fb[3 + u];
+        }
+        q.pp = 1;
+        launch_e3d_general_pdl<float>(q, J->stream);
+        launch_step3d_fused(q, J->fmaps[0], J->stream);
+        q.ex = q.exo; q.ey = q.eyo; q.ez = q.ezo;
+        launch_h3d_general_pdl<float>(q, J->stream);
+        return;
+      }
+    }
     run_parts<T>(J, p, parts, true, true);
     run_parts<T>(J, p, parts, false, true);
   };
+  int from = 0;
   auto cores = [&](int c) {
     if constexpr (sizeof(T) == 4) {
       if (J->dim == 2 && c == fused_tile(J)) {
         StepParams<float> q = p;
         block_buffers(J, q, pl, 0);
         launch_blocks(J, q, pl);
+        return;
+      }
+      if (J->dim == 3 && c == kBlock3Tile) {
+        StepParams<float> q = p;
+        Block3 b3;
+        block3_buffers(J, q, b3, from ^= 1);  // to and fro, as steps run
+        launch_blocks3(J, q, b3, 2);
         return;
       }
       if (J->dim == 3 && c == fused_tile(J)) {
@@ -2082,11 +2292,19 @@ int tune_tiles(fdtd_job *J) {
     float ms = 0.f;
     return cudaEventSynchronize(b) == cudaSuccess && cudaEventElapsedTime(&ms, a, b) == cudaSuccess ? ms : 3.0e38f;
   };
-  for (int c = 0; c < nshapes; ++c) {
-    const bool block = J->dim == 2 && c == fused_tile(J);
+  const int last = J->block3_ok ? kBlock3Tile : nshapes - 1;
+  for (int c = 0; c <= last; ++c) {
+    if (c >= nshapes && c < kBlock3Tile) continue;
+    const bool block = (J->dim == 2 && c == fused_tile(J)) || (J->dim == 3 && c == kBlock3Tile);
     if (block) best = time5(split_step);
     p.tile = c;
-    const float ms = time5([&] { cores(c); }) / (block ? (float)pl.ks : 1.f);  // of a step
+    float ms = time5([&] { cores(c); }) / (block ? (float)(J->dim == 2 ? pl.ks : 2) : 1.f);  // of a step
+    // (the first runs of the 3D block-step kernel take a quarter longer than all later ones)
+    if (J->dim == 3 && block) ms = std::min(ms, time5([&] { cores(c); }) / 2.f);
+    if (J->dim == 3 && c < fused_tile(J) && ms < best_split) {
+      best_split = ms;
+      J->split_tile = c;
+    }
     if (ms < best) {
       best = ms;
       choice = c;
@@ -2097,7 +2315,7 @@ int tune_tiles(fdtd_job *J) {
   CK(cudaGetLastError());
   J->tile = choice;
   std::lock_guard<std::mutex> lk(g_tune_mu);
-  g_tune[key] = choice;
+  g_tune[key] = choice | J->split_tile << 8;
   return FDTD_OK;
 }
 
@@ -2168,7 +2386,8 @@ int after_sample(fdtd_job *J, int n) {
 
 // A job steps through a fused step kernel when the tuner (or fdtd_set_tile)
 // chose it.  The per-procedure entry points keep the split kernels.
-bool fused_mode(const fdtd_job *J) { return J->fused_ok && J->tile == fused_tile(J); }
+bool block3_mode(const fdtd_job *J) { return J->block3_ok && J->tile == kBlock3Tile; }
+bool fused_mode(const fdtd_job *J) { return (J->fused_ok && J->tile == fused_tile(J)) || block3_mode(J); }
 
 // k steps (at most the plan's) of the 2D block-step kernel in one launch, from
 // field set pp to the other; it takes the samples of each step itself.
@@ -2190,6 +2409,41 @@ int block_step(fdtd_job *J, int n, int k, int slot, bool graph) {
   if (!graph) ev_record(J, FDTD_KERNEL_STEP, false);
   if (ran < 0) return FDTD_ECUDA;
   J->launches += ran;
+  J->pp ^= 1;
+  J->prog_prev = -1;
+  CK(cudaGetLastError());
+  return FDTD_OK;
+}
+
+// k steps (1 or 2) of the 3D block-step kernel in one launch, then their samples
+int block3_step(fdtd_job *J, int n, int k, int slot, bool graph) {
+  StepParams<float> p;
+  fill_common<float>(J, p);
+  set_sources<float>(J, p);
+  p.n = n;
+  p.slot = slot;
+  ring_params(J, p, graph);
+  Block3 b;
+  block3_buffers(J, p, b, J->pp);
+  if (!graph) ev_record(J, FDTD_KERNEL_STEP, true);
+  const int ran = launch_blocks3(J, p, b, k);
+  if (!graph) ev_record(J, FDTD_KERNEL_STEP, false);
+  if (ran < 0) return FDTD_ECUDA;
+  J->launches += ran;
+  // the samples: of the first of two steps from the rows kept, of the last from
+  // the new fields
+  if (k == 2 && b.seg) {
+    p.first = b.first;
+    p.seg = b.seg;
+    p.seg_nt = b.ntx;
+    p.seg_ox = b.ox;
+    J->launches += launch_gather<float>(p, J->stream);
+  }
+  p.seg = nullptr;
+  p.slot = slot + k - 1;
+  p.n = n + k - 1;
+  p.ex = p.exo; p.ey = p.eyo; p.ez = p.ezo; p.hx = p.hxo; p.hy = p.hyo; p.hz = p.hzo;
+  J->launches += launch_gather<float>(p, J->stream);
   J->pp ^= 1;
   J->prog_prev = -1;
   CK(cudaGetLastError());
@@ -2258,6 +2512,8 @@ int fused_settle(fdtd_job *J) {
   for (int c = 0; c < 6; ++c)
     if (J->Fb[c]) CK(cudaMemcpyAsync(J->F[c], J->Fb[c], bytes, cudaMemcpyDeviceToDevice, J->stream));
   if (J->spb) CK(cudaMemcpyAsync(J->d_sp[0], J->spb, bytes, cudaMemcpyDeviceToDevice, J->stream));
+  for (int q = 0; q < 6; ++q)
+    if (J->spb3[q]) CK(cudaMemcpyAsync(J->d_sp[q], J->spb3[q], bytes, cudaMemcpyDeviceToDevice, J->stream));
   if (J->ade_b) CK(cudaMemcpyAsync(J->d_ade_state, J->ade_b, ade_bytes(J), cudaMemcpyDeviceToDevice, J->stream));
   J->pp = 0;
   J->prog_prev = -1;
@@ -2269,15 +2525,20 @@ template <typename T>
 int eager_steps(fdtd_job *J, int n, int left, int *done) {
   int rc;
   *done = 1;
-  if (fused_mode(J) && J->dim == 2) {  // as many as a launch takes and the sample ring has room for
-    const int k = std::min(std::min(left, J->blk.ks), kStageSteps - J->stage_fill);
-    if ((rc = block_step(J, n, k, J->stage_fill, false))) return rc;
+  // as many steps as a launch takes and the sample ring has room for; a single
+  // step of the 3D block-step kernel only to come back to the canonical field
+  // set (512^3: 2.1 ms against 1.7 split; the 256 x 256 x 384 column 0.36 and 0.30)
+  const int most = J->dim == 2 ? J->blk.ks : 2;
+  const int k = std::min(std::min(left, most), kStageSteps - J->stage_fill);
+  const bool block = fused_mode(J) && (J->dim == 2 || block3_mode(J));
+  if (block && (J->dim == 2 || k > 1 || J->pp)) {
+    if ((rc = J->dim == 2 ? block_step(J, n, k, J->stage_fill, false) : block3_step(J, n, k, J->stage_fill, false))) return rc;
     for (int s = 0; s < k; ++s)
       if ((rc = after_sample<T>(J, n + s))) return rc;
     *done = k;
     return FDTD_OK;
   }
-  if (fused_mode(J)) {
+  if (fused_mode(J) && !block) {
     if ((rc = fused_step<T>(J, n, J->stage_fill, false))) return rc;
     return after_sample<T>(J, n);
   }
@@ -2335,6 +2596,10 @@ int ring_graph(fdtd_job *J) {
     if (fused_mode(J) && J->dim == 2) {
       bad = block_step(J, 0, J->blk.ks, s, true);
       s += J->blk.ks - 1;
+      continue;
+    }
+    if (block3_mode(J)) {
+      bad = block3_step(J, 0, 2, s++, true);
       continue;
     }
     if (fused_mode(J)) {
@@ -2584,6 +2849,17 @@ int step_impl(fdtd_job *J, int n_first, int n_steps) {
   // finish a partly filled ring eagerly, replay whole rings from the graph,
   // run the tail eagerly (the per-launch events of fdtd_profile need eager)
   int k = 0;
+  // A replay starts from the canonical field set, and bringing the fields there
+  // is a copy (512^3: 1.9 ms).  So before and after replays the 3D block-step
+  // kernel runs an even number of two-step launches, and split steps, which
+  // update in place, take the rest (512^3: 1700 us a step).
+  auto even_tail = [&](int rest) -> int {
+    for (; block3_mode(J) && rest > 0 && (rest % 4 != 0 || J->pp); --rest, ++n)
+      if (const int e = eager_steps<T>(J, n, 1, &k)) return e;
+    return FDTD_OK;
+  };
+  const bool replays = J->use_graph && !J->prof && end - n - (kStageSteps - J->stage_fill) % kStageSteps >= kStageSteps;
+  if (replays && J->stage_fill != 0 && (rc = even_tail(kStageSteps - J->stage_fill))) return rc;
   for (; n < end && J->stage_fill != 0; n += k)
     if ((rc = eager_steps<T>(J, n, end - n, &k))) return rc;
   if (J->use_graph && !J->prof && end - n >= kStageSteps) {
@@ -2593,10 +2869,11 @@ int step_impl(fdtd_job *J, int n_first, int n_steps) {
       n += kStageSteps;
     }
     if ((rc = flush_fold<T>(J))) return rc;
+    if ((rc = even_tail(end - n))) return rc;
   }
   for (; n < end; n += k)
     if ((rc = eager_steps<T>(J, n, end - n, &k))) return rc;
-  return J->dim == 3 ? fused_settle(J) : FDTD_OK;
+  return J->dim == 3 && !block3_mode(J) ? fused_settle(J) : FDTD_OK;
 }
 
 #define DISPATCH(J, call) ((J)->g.precision == FDTD_F32 ? call<float> : call<double>)
@@ -2939,6 +3216,11 @@ int fdtd::pack_run(fdtd::Pack *P, int rings, cudaEvent_t done) {
 }
 
 // =========================================================================
+int fdtd::make_lean(fdtd_job *J, uint64_t *est) {
+  J->lean = true;
+  return fdtd_estimate_bytes(J, est);
+}
+
 extern "C" {
 
 int fdtd_last_error(char *buf, size_t len) {
@@ -3556,21 +3838,37 @@ int fdtd_estimate_bytes(const fdtd_job *J, uint64_t *bytes) {
   const int nx = J->nx, ny = J->ny, nz = J->nz;
   uint64_t b = N * w * (J->dim == 3 ? 6 : J->dim == 2 ? 3 : 2) + N;  // fields, material ids
   // the fused 3D step kernel's second set of fields (commit may give it back)
-  if (J->dim == 3 && w == 4 && J->nx % 4 == 0 && !J->has_tfbox &&
-      !(J->has_pml && J->pml.mode == FDTD_PML_REFERENCE))
-    b += 6 * N * w;
+  const bool block3 = J->dim == 3 && w == 4 && J->nx % 4 == 0 && !J->has_tfbox && !J->lean &&
+                      !(J->has_pml && J->pml.mode == FDTD_PML_REFERENCE);
+  if (block3) b += 6 * N * w;
+  // the 3D block-step kernel's: the stored PML parts, row flags and segments of
+  // the columns of tiles (60 cells), the tiles' order
+  if (block3) {
+    const uint64_t col = (uint64_t)(nx + 59) / 60;
+    b += (J->has_pml ? 6 * N * w : 0) + (uint64_t)ny * nz * col * 5 + col * ((uint64_t)ny / 13 + 1) * ((uint64_t)nz / 8 + 1) * 4;
+    for (auto &M : J->mons)
+      b += (uint64_t)(M.d.hi[1] - M.d.lo[1] + 1) * (M.d.hi[2] - M.d.lo[2] + 1) * ((M.d.hi[0] - M.d.lo[0]) / 60 + 2) * 360 * w;
+    b += J->probes.size() * 360ull * w;
+  }
   // the 2D block-step kernel's: the fields and the stored PML part, its tiles
   // (at least 112 x 16 cells, 96 bytes with their flags)
-  const bool block2 = J->dim == 2 && w == 4 && !J->has_tfbox && !(J->has_pml && J->pml.mode == FDTD_PML_REFERENCE);
+  const bool block2 = J->dim == 2 && w == 4 && !J->has_tfbox && !J->lean && !(J->has_pml && J->pml.mode == FDTD_PML_REFERENCE);
   if (block2) b += 4 * N * w + ((uint64_t)nx / 112 + 1) * ((uint64_t)ny / 16 + 1) * 96;
-  if (J->dim == 1)  // the 1D block-step kernel's second set and slot map
+  if (J->dim == 1 && !J->lean)  // the 1D block-step kernel's second set and slot map
     b += (J->has_tfsf ? 4 : 2) * N * w + 4 * N + 8ull * (J->pml.npml[1][0] + 2) * w;
   if (J->has_tfsf) b += 2 * N * w;
   if (J->has_tfbox) b += 2ull * ny * w + 4 * w;
   // dispersive cells: each region's cells, bounded per sphere / box
   uint64_t nade = 0;
+  int alo[3] = {INT32_MAX, INT32_MAX, INT32_MAX}, ahi[3] = {-1, -1, -1};  // the box of them all
   for (auto &m : J->mats) {
     if (!is_ade_kind(m.kind)) continue;
+    int blo[3], bhi[3];
+    region_bounds(J, m, blo, bhi);
+    for (int a = 0; a < 3; ++a) {
+      alo[a] = std::min(alo[a], blo[a]);
+      ahi[a] = std::max(ahi[a], bhi[a]);
+    }
     if (m.region.kind == FDTD_REGION_MASK) {
       for (uint8_t v : m.mask) nade += v != 0;
     } else if (m.region.kind == FDTD_REGION_SPHERES) {
@@ -3595,7 +3893,13 @@ int fdtd_estimate_bytes(const fdtd_job *J, uint64_t *bytes) {
   b += nade * ((uint64_t)nf * 3 * w + 5) + 32ull * nf * 3 * w;
   // and its dispersive cells: a second state, and in up to four tiles a list
   // entry and the scratch state
-  if (J->dim == 1) b += nade * (uint64_t)nf * 3 * w + 32ull * nf * 3 * w;
+  if (J->dim == 1 && !J->lean) b += nade * (uint64_t)nf * 3 * w + 32ull * nf * 3 * w;
+  if (block3 && nade > 0) {  // two more states, and the slots over the box
+    b += 2 * (nade * (uint64_t)nf * 3 * w + 32ull * nf * 3 * w);
+    uint64_t box = 4;
+    for (int a = 0; a < 3; ++a) box *= (uint64_t)std::max(1, ahi[a] - alo[a] + 1);
+    b += std::min(box, 4 * N);
+  }
   if (block2) b += nade * ((uint64_t)nf * 3 * w + 4 * (8 + 2ull * nf * w)) + 32ull * nf * 3 * w;
   if (J->has_pml && J->pml.mode == FDTD_PML_SPLIT) {
     b += (uint64_t)(J->dim == 3 ? 6 : 1) * (w == 8 ? 2 : 1) * N * w;
@@ -3669,7 +3973,7 @@ int fdtd_kernel_cells(const fdtd_job *J, int32_t kind, int64_t *cells) {
   int64_t c = 0;
   if (kind == FDTD_KERNEL_E || kind == FDTD_KERNEL_H) c = J->dim >= 2 ? (int64_t)J->ncore * J->vec : 0;
   else if (kind == FDTD_KERNEL_STEP)
-    c = !fused_mode(J) ? 0 : J->dim == 3 ? (int64_t)J->ncore * J->vec : (int64_t)J->ncell;
+    c = !fused_mode(J) ? 0 : J->dim == 3 && !block3_mode(J) ? (int64_t)J->ncore * J->vec : (int64_t)J->ncell;
   else if (kind == FDTD_KERNEL_EDGE)
     c = J->dim >= 2 ? (int64_t)J->nedge * J->vec : 0;
   else if (kind == FDTD_KERNEL_ADE) c = J->dim == 2 ? J->nade : 0;

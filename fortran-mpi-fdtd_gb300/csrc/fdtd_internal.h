@@ -23,6 +23,8 @@
 
 #include "fdtd_gb300.h"
 
+struct fdtd_job;
+
 namespace fdtd {
 
 // tensor maps of one buffer's H arrays for the fused 3D step kernel: one-plane
@@ -220,6 +222,9 @@ struct StepParams {
   int vec;                 // cells per thread along x in the 2D tile path
   double *mean_part;       // mean monitors: FP64 partial sums per block
   unsigned *mean_ctr;      // mean monitors: blocks done per component
+  const T *first;          // gather: rows of the field values (k3b.cu), [seg[row*seg_nt + i/seg_ox]]
+  const int *seg;          //   [component][i % seg_ox]; null: the values are the fields'
+  int seg_nt, seg_ox;
   // 2D/3D total-field/scattered-field box (plane wave along +y)
   int tf_on;
   int tf_lo[3], tf_hi[3];  // total-field box, inclusive cells
@@ -344,6 +349,26 @@ int launch_step3d_fused(const StepParams<float> &p, const FusedMaps &m, void *st
 // blocks and dynamic shared memory of one launch
 void step3d_fused_shape(const StepParams<float> &p, int *blocks, int *smem);
 
+// ---- the 3D block-step kernel (k3b.cu, FP32): two steps of the grid per launch
+struct Block3 {
+  int ox, oy, oz;         // cells, rows and planes that a tile owns
+  int ntx, nty, ntz;      // tiles
+  const uint8_t *flags;   // per x-row and column of tiles: sources, samples, materials, general cells (B3_*)
+  const int *order;       // tiles in the order of launch, those with dispersive cells first
+  int nade;               // how many have
+  float *spo[6];          // where the stored PML parts of the new step go
+  float *ade_mid, *ade_out;  // dispersive state after the first and the last step
+  const int *slot;        // slots of the dispersive cells over the box alo.. of an[] cells
+  int alo[3], an[3];
+  int one_gold;           // every dispersive cell is of one gold material
+  float *first;           // rows with samples after the first step, [segment][component][cell of the tile's row]
+  const int *seg;         // segment of a row of a column of tiles
+};
+void block3_tiles(Block3 &b, int nx, int ny, int nz, int num_sms);
+void launch_row_flags3(const StepParams<float> &p, const Block3 &b, uint8_t *out, void *stream);
+// the tiles with dispersive cells or those without; returns the kernels launched, -1 on failure
+int launch_step3d_block(const StepParams<float> &p, const Block3 &b, int steps, bool ade, void *stream);
+
 // separate gather (per-procedure API, or monitors inside reference slabs)
 // returns the kernels launched
 template <typename T> int launch_gather(const StepParams<T> &p, void *stream);
@@ -372,6 +397,9 @@ struct DftParams {
   long long stage_row;
   int total_work_blocks;
 };
+// leave the kernels that need second sets of buffers out of an uncommitted job,
+// and estimate again (fdtd_server.cu: a job that would not fit with them)
+int make_lean(fdtd_job *job, uint64_t *est);
 template <typename T> void launch_dft(const DftParams &d, const T *stage, void *stream);
 // every ring of a line's stage in one launch, for monitors of few samples
 // (dft_rings_fit); d.nslots: the rows of all of them.  Returns the launches.

@@ -111,6 +111,7 @@ void finish(fdtd_server *S, Req *r, int rc, const char *why) {
 void admit(fdtd_server *S) {
   while (!S->queue.empty() && (int)S->active.size() + S->committing < S->d.max_active && !S->stop) {
     Req *r = S->queue.front();
+    if (r->est > S->budget) fdtd::make_lean(r->job, &r->est);  // without what only speeds it up
     if (r->est > S->budget) {
       S->queue.pop_front();
       finish(S, r, FDTD_ENOMEM, "job footprint exceeds the server's HBM budget");

@@ -223,6 +223,14 @@ template int preload_dft<double>();
 
 constexpr int kMeanThreads = 256;  // threads per block of the gather launch
 
+// a field value from the rows that a step kernel kept (StepParams::first)
+template <typename T>
+__device__ __forceinline__ T first_value(const StepParams<T> &p, int comp, int i, int j, int k) {
+  const int tx = i / p.seg_ox;
+  const long long s = __ldg(p.seg + ((long long)k * p.ny + j) * p.seg_nt + tx);
+  return p.first[(s * 6 + comp) * p.seg_ox + (i - tx * p.seg_ox)];
+}
+
 // Stand-alone gather of the monitored cells and probes after the H update:
 // one thread per monitored (component, cell) sample, plus one per probe.
 template <typename T>
@@ -242,7 +250,8 @@ __device__ __forceinline__ void gather_cells(const StepParams<T> &p, long long t
       const int k = m.lo[2] + (int)(c / ((long long)wx * wy));
       const long long cell = (long long)i + (long long)p.nx * (j + (long long)p.ny * k);
       const T *f = F[m.comps[u]];
-      stage_ring(p)[(long long)p.slot * p.stage_row + m.base + t] = f ? f[cell] : T(0);
+      stage_ring(p)[(long long)p.slot * p.stage_row + m.base + t] =
+          p.seg ? first_value(p, m.comps[u], i, j, k) : f ? f[cell] : T(0);
       return;
     }
     t -= ns;
@@ -255,7 +264,8 @@ __device__ __forceinline__ void gather_cells(const StepParams<T> &p, long long t
     const long long cell = (long long)pr.cell[0] + (long long)p.nx * (pr.cell[1] + (long long)p.ny * pr.cell[2]);
     for (int u = 0; u < pr.ncomp; ++u) {
       const T *f = F[pr.comps[u]];
-      pr.buf[st * pr.ncomp + u] = f ? (double)f[cell] : 0.0;
+      pr.buf[st * pr.ncomp + u] =
+          p.seg ? (double)first_value(p, pr.comps[u], pr.cell[0], pr.cell[1], pr.cell[2]) : f ? (double)f[cell] : 0.0;
     }
   }
 }
@@ -300,7 +310,8 @@ __device__ __forceinline__ void gather_mean(const StepParams<T> &p, int b) {
         if (e < ne) {
           const int r = r0 + e / wx, i = e % wx;
           const int j = m.lo[1] + r % wy, k = m.lo[2] + r / wy;
-          v[q8] = f[(long long)(m.lo[0] + i) + (long long)p.nx * (j + (long long)p.ny * k)];
+          v[q8] = p.seg ? first_value(p, m.comps[u], m.lo[0] + i, j, k)
+                        : f[(long long)(m.lo[0] + i) + (long long)p.nx * (j + (long long)p.ny * k)];
         }
       }
 #pragma unroll

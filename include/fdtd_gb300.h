@@ -442,8 +442,8 @@ int fdtd_estimate_bytes(const fdtd_job *job, uint64_t *bytes);
  * FDTD_KERNEL_ADE: no launch of its own any more (the split 2D step appends
  * the dispersive cells' blocks to its E edge kernel, timed as
  * FDTD_KERNEL_EDGE); FDTD_KERNEL_STEP: the fused 3D step kernel (E and H of
- * the core box in one launch) and the 2D block-step kernels (the whole grid,
- * up to eight steps in one timed pair of launches). */
+ * the core box in one launch) and the block-step kernels (the whole grid, up
+ * to eight steps in 2D and two in 3D, in one timed pair of launches). */
 enum { FDTD_KERNEL_E = 0, FDTD_KERNEL_H = 1, FDTD_KERNEL_DFT = 2, FDTD_KERNEL_LINE1D = 3,
        FDTD_KERNEL_EDGE = 4, FDTD_KERNEL_ADE = 5, FDTD_KERNEL_STEP = 6, FDTD_KERNEL_COUNT = 7 };
 int fdtd_profile(fdtd_job *job, int32_t enable);
@@ -468,9 +468,15 @@ int fdtd_kernel_time(fdtd_job *job, int32_t kind, int64_t *launches, double *ms)
  * which takes E and H of the core box from step n to n+1 in one pass over
  * two sets of field buffers used in turn (the job then holds a second copy
  * of its six field arrays); pinning one elsewhere fails at commit with
- * FDTD_EINVAL.  Results do not depend on the shape.  Environment FDTD_NO_TMA
- * leaves the TMA-staged kernels out, FDTD_NO_FUSED the fused ones.
- * fdtd_get_tile returns the shape in use (0: the job has no core kernels). */
+ * FDTD_EINVAL.  The tuner also offers the 3D block-step kernel (two steps of
+ * the whole grid per launch; FP32, 4-cell vectors, periodic or not, no
+ * reference slabs or TFSF box; second copies of the six fields, the stored
+ * PML parts and the dispersive state, and none if the device has no room for
+ * them); it cannot be pinned, but environment FDTD_TUNE=block takes it
+ * wherever it is offered.  Results do not depend on the shape.  Environment
+ * FDTD_NO_TMA leaves the TMA-staged kernels out, FDTD_NO_FUSED the fused and
+ * block-step ones.  fdtd_get_tile returns the shape in use (0: the job has no
+ * core kernels; 10: the 3D block-step kernel). */
 int fdtd_set_tile(fdtd_job *job, int32_t tile);
 int fdtd_get_tile(const fdtd_job *job, int32_t *tile);
 /* Cells one launch of kernel class `kind` updates (FDTD_KERNEL_DFT: monitored
