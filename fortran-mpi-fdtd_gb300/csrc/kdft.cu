@@ -330,10 +330,22 @@ __device__ __forceinline__ void gather_mean(const StepParams<T> &p, int b) {
     last = atomicAdd(p.mean_ctr + slot, 1u) == (unsigned)(m.mchunks - 1);
   }
   __syncthreads();
-  if (last && threadIdx.x == 0) {
-    __threadfence();
-    double tot = 0.0;
-    for (int c = 0; c < m.mchunks; ++c) tot += __ldcg(p.mean_part + slot + c);
+  if (!last) return;
+  __threadfence();
+  // the partial sums come a block's width at a time, and are added in block
+  // order (one thread loading each in turn: 3 us a step more on the column of
+  // 65536-cell planes)
+  __shared__ double fin[kMeanThreads];
+  double tot = 0.0;
+  for (int c0 = 0; c0 < m.mchunks; c0 += kMeanThreads) {
+    const int nc = min(kMeanThreads, m.mchunks - c0);
+    if ((int)threadIdx.x < nc) fin[threadIdx.x] = __ldcg(p.mean_part + slot + c0 + threadIdx.x);
+    __syncthreads();
+    if (threadIdx.x == 0)
+      for (int c = 0; c < nc; ++c) tot += fin[c];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
     stage_ring(p)[(long long)p.slot * p.stage_row + m.base + u] = T(tot / (double)m.boxcells);
     p.mean_ctr[slot] = 0u;
   }
