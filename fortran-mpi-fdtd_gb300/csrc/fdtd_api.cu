@@ -1906,6 +1906,11 @@ int ensure_srctab(fdtd_job *J, int n_max) {
     cudaError_t e = pool_alloc(J, (void **)&nb, (size_t)cap * nsrc * sizeof(double));
     if (e != cudaSuccess) return set_err(FDTD_ENOMEM, "source table: %s", cudaGetErrorString(e));
   }
+  // Whole pieces of kSrcPiece steps at a time: a caller that steps one by one, or
+  // through the per-procedure calls, would otherwise wait every step for the copy
+  // of one value behind everything in flight (512^2: 15 of 34 us a step).
+  constexpr long long kSrcPiece = 256;
+  n_max = (int)std::min<long long>(std::min<long long>(cap, INT32_MAX), ((long long)n_max + kSrcPiece - 1) / kSrcPiece * kSrcPiece);
   for (long long n = old_steps + 1; n <= n_max; ++n) {
     const double t = (double)(n - 1) * J->g.dt;           // t=real(n-1,8)*dt
     for (auto &s : J->srcs)
