@@ -271,7 +271,7 @@ def config_runs(stream):
     l32, l64 = timed(o32, 2000, 18000, lambda w: 4 * w + 1), timed(o64, 2000, 18000, lambda w: 4 * w + 1)
     for r in (l32, l64):
         r["steps_per_s"] = 1e3 / r["ms_per_step"]
-        r["note"] = "4000 cells: one persistent block, latency-bound; the roofline does not apply"
+        r["note"] = "4000 cells: a launch per 32 steps (FP64: 16), latency-bound; the roofline does not apply"
     out["1d_gold_slab_4000"] = {"fp32": l32, "fp64_plain": l64}
     return out
 
