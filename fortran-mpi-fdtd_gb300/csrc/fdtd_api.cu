@@ -2438,13 +2438,9 @@ int block3_step(fdtd_job *J, int n, int k, int slot, bool graph) {
   // the samples: of the first of two steps from the rows kept, of the last from
   // the new fields
   if (k == 2 && b.seg) {
-    p.first = b.first;
-    p.seg = b.seg;
-    p.seg_nt = b.ntx;
-    p.seg_ox = b.ox;
-    J->launches += launch_gather<float>(p, J->stream);
+    const KeptRows kept{b.first, b.seg, b.ntx, b.ox};
+    J->launches += launch_gather<float>(p, J->stream, &kept);
   }
-  p.seg = nullptr;
   p.slot = slot + k - 1;
   p.n = n + k - 1;
   p.ex = p.exo; p.ey = p.eyo; p.ez = p.ezo; p.hx = p.hxo; p.hy = p.hyo; p.hz = p.hzo;

@@ -222,9 +222,6 @@ struct StepParams {
   int vec;                 // cells per thread along x in the 2D tile path
   double *mean_part;       // mean monitors: FP64 partial sums per block
   unsigned *mean_ctr;      // mean monitors: blocks done per component
-  const T *first;          // gather: rows of the field values (k3b.cu), [seg[row*seg_nt + i/seg_ox]]
-  const int *seg;          //   [component][i % seg_ox]; null: the values are the fields'
-  int seg_nt, seg_ox;
   // 2D/3D total-field/scattered-field box (plane wave along +y)
   int tf_on;
   int tf_lo[3], tf_hi[3];  // total-field box, inclusive cells
@@ -371,7 +368,14 @@ int launch_step3d_block(const StepParams<float> &p, const Block3 &b, int steps, 
 
 // separate gather (per-procedure API, or monitors inside reference slabs)
 // returns the kernels launched
-template <typename T> int launch_gather(const StepParams<T> &p, void *stream);
+// kept: null, or where the values come from instead of the fields: rows that a
+// step kernel kept, [seg[row*nt + i/ox]][component][i % ox]
+struct KeptRows {
+  const float *first;
+  const int *seg;
+  int nt, ox;
+};
+template <typename T> int launch_gather(const StepParams<T> &p, void *stream, const KeptRows *kept = nullptr);
 // total-field/scattered-field box: incident line and face terms of a half step
 // kcheck.cu: count the non-finite float (esz 4) or double (esz 8) values of a buffer
 int launch_count_nonfinite(const void *p, size_t bytes, int esz, unsigned long long *out, int num_sms, void *stream);

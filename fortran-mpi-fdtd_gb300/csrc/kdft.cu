@@ -223,18 +223,24 @@ template int preload_dft<double>();
 
 constexpr int kMeanThreads = 256;  // threads per block of the gather launch
 
-// a field value from the rows that a step kernel kept (StepParams::first)
+struct GatherArgs {
+  int cell_blocks;
+  KeptRows kept;
+};
+
+// a field value from the rows that a step kernel kept
 template <typename T>
-__device__ __forceinline__ T first_value(const StepParams<T> &p, int comp, int i, int j, int k) {
-  const int tx = i / p.seg_ox;
-  const long long s = __ldg(p.seg + ((long long)k * p.ny + j) * p.seg_nt + tx);
-  return p.first[(s * 6 + comp) * p.seg_ox + (i - tx * p.seg_ox)];
+__device__ __forceinline__ T first_value(const StepParams<T> &p, const KeptRows &r, int comp, int i, int j, int k) {
+  const int tx = i / r.ox;
+  const long long s = __ldg(r.seg + ((long long)k * p.ny + j) * r.nt + tx);
+  return r.first[(s * 6 + comp) * r.ox + (i - tx * r.ox)];
 }
 
 // Stand-alone gather of the monitored cells and probes after the H update:
 // one thread per monitored (component, cell) sample, plus one per probe.
-template <typename T>
-__device__ __forceinline__ void gather_cells(const StepParams<T> &p, long long t) {
+// KEPT: the values come from kept rows
+template <typename T, bool KEPT>
+__device__ __forceinline__ void gather_cells(const StepParams<T> &p, const GatherArgs &g, long long t) {
   const int n = step_n(p);
   const T *F[6] = {p.ex, p.ey, p.ez, p.hx, p.hy, p.hz};
   for (int q = 0; q < p.nmon; ++q) {
@@ -251,7 +257,7 @@ __device__ __forceinline__ void gather_cells(const StepParams<T> &p, long long t
       const long long cell = (long long)i + (long long)p.nx * (j + (long long)p.ny * k);
       const T *f = F[m.comps[u]];
       stage_ring(p)[(long long)p.slot * p.stage_row + m.base + t] =
-          p.seg ? first_value(p, m.comps[u], i, j, k) : f ? f[cell] : T(0);
+          KEPT ? first_value(p, g.kept, m.comps[u], i, j, k) : f ? f[cell] : T(0);
       return;
     }
     t -= ns;
@@ -265,7 +271,7 @@ __device__ __forceinline__ void gather_cells(const StepParams<T> &p, long long t
     for (int u = 0; u < pr.ncomp; ++u) {
       const T *f = F[pr.comps[u]];
       pr.buf[st * pr.ncomp + u] =
-          p.seg ? (double)first_value(p, pr.comps[u], pr.cell[0], pr.cell[1], pr.cell[2]) : f ? (double)f[cell] : 0.0;
+          KEPT ? (double)first_value(p, g.kept, pr.comps[u], pr.cell[0], pr.cell[1], pr.cell[2]) : f ? (double)f[cell] : 0.0;
     }
   }
 }
@@ -279,8 +285,8 @@ __device__ __forceinline__ void gather_cells(const StepParams<T> &p, long long t
 // block order, stages the mean as the component's one sample and resets the
 // counter.  The result depends on neither which block finishes last nor
 // timing.
-template <typename T>
-__device__ __forceinline__ void gather_mean(const StepParams<T> &p, int b) {
+template <typename T, bool KEPT>
+__device__ __forceinline__ void gather_mean(const StepParams<T> &p, const GatherArgs &g, int b) {
   __shared__ double part[kMeanThreads / 32];
   __shared__ int last;
   int q = 0;
@@ -310,7 +316,7 @@ __device__ __forceinline__ void gather_mean(const StepParams<T> &p, int b) {
         if (e < ne) {
           const int r = r0 + e / wx, i = e % wx;
           const int j = m.lo[1] + r % wy, k = m.lo[2] + r / wy;
-          v[q8] = p.seg ? first_value(p, m.comps[u], m.lo[0] + i, j, k)
+          v[q8] = KEPT ? first_value(p, g.kept, m.comps[u], m.lo[0] + i, j, k)
                         : f[(long long)(m.lo[0] + i) + (long long)p.nx * (j + (long long)p.ny * k)];
         }
       }
@@ -355,16 +361,16 @@ __device__ __forceinline__ void gather_mean(const StepParams<T> &p, int b) {
 // the rest reduce the mean monitors.  It follows the H half step with a
 // programmatic dependency and releases the next kernel at once, so the next
 // E half's launch overlaps it.
-template <typename T>
-__global__ void __launch_bounds__(kMeanThreads) gather_kernel(const __grid_constant__ StepParams<T> p, int cell_blocks) {
+template <typename T, bool KEPT, bool MEAN>
+__global__ void __launch_bounds__(kMeanThreads) gather_kernel(const __grid_constant__ StepParams<T> p, const __grid_constant__ GatherArgs g) {
   pdl_wait();
   pdl_release();
-  if ((int)blockIdx.x < cell_blocks) gather_cells<T>(p, (long long)blockIdx.x * kMeanThreads + threadIdx.x);
-  else gather_mean<T>(p, (int)blockIdx.x - cell_blocks);
+  if (!MEAN || (int)blockIdx.x < g.cell_blocks) gather_cells<T, KEPT>(p, g, (long long)blockIdx.x * kMeanThreads + threadIdx.x);
+  else if (MEAN) gather_mean<T, KEPT>(p, g, (int)blockIdx.x - g.cell_blocks);
 }
 
 template <typename T>
-int launch_gather(const StepParams<T> &p, void *stream) {
+int launch_gather(const StepParams<T> &p, void *stream, const KeptRows *kept) {
   long long total = p.nprobe;
   int nmean = 0;
   for (int q = 0; q < p.nmon; ++q) {
@@ -373,11 +379,15 @@ int launch_gather(const StepParams<T> &p, void *stream) {
   }
   const int cell_blocks = (int)((total + kMeanThreads - 1) / kMeanThreads);
   if (cell_blocks + nmean <= 0) return 0;
-  launch_pdl2(gather_kernel<T>, cell_blocks + nmean, kMeanThreads, (cudaStream_t)stream, p, cell_blocks);
+  GatherArgs g{cell_blocks, {}};
+  if (kept) g.kept = *kept;
+  auto launch = [&](auto kernel) { launch_pdl2(kernel, cell_blocks + nmean, kMeanThreads, (cudaStream_t)stream, p, g); };
+  if (kept) nmean ? launch(gather_kernel<T, true, true>) : launch(gather_kernel<T, true, false>);
+  else nmean ? launch(gather_kernel<T, false, true>) : launch(gather_kernel<T, false, false>);
   return 1;
 }
 
-template int launch_gather<float>(const StepParams<float> &, void *);
-template int launch_gather<double>(const StepParams<double> &, void *);
+template int launch_gather<float>(const StepParams<float> &, void *, const KeptRows *);
+template int launch_gather<double>(const StepParams<double> &, void *, const KeptRows *);
 
 }  // namespace fdtd
