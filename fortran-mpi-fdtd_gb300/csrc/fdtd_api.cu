@@ -3724,6 +3724,7 @@ int fdtd_load_state(fdtd_job *J, const void *buf, uint64_t bytes) {
     if (b) CK(cudaMemcpyAsync(P.buf, o, b, cudaMemcpyHostToDevice, J->stream));
     o += b;
   }
+  CK(cudaStreamSynchronize(J->stream));  // the caller may reuse buf
   J->stage_fill = h.stage_fill;
   J->stage_half = h.stage_half & 1;
   J->fold_pending = false;
