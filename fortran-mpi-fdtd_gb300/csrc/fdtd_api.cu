@@ -3710,8 +3710,8 @@ int fdtd_load_state(fdtd_job *J, const void *buf, uint64_t bytes) {
   if (expect != bytes) return set_err(FDTD_EINVAL, "checkpoint of %llu bytes, its tables describe %llu",
                                       (unsigned long long)bytes, (unsigned long long)expect);
   CK(cudaStreamSynchronize(J->stream));
-  J->pp = 0;  // the loaded state goes to the canonical buffers
   if (n_probe_max > 0 && (rc = ensure_probe_cap(J, n_probe_max))) return rc;
+  J->pp = 0;  // the loaded state goes to the canonical buffers
   const char *o = pr + J->probes.size() * 2 * sizeof(int32_t);
   for (auto &s : J->state) {
     CK(cudaMemcpyAsync(s.p, o, s.bytes, cudaMemcpyHostToDevice, J->stream));

@@ -41,3 +41,38 @@ def test_load_state_leaves_the_callers_buffer_free(gpu):
         pinned[tail:] = 0x3f
         np.testing.assert_array_equal(J.save_state(), want)
     J.close()
+
+
+def test_refused_load_state_leaves_the_state(gpu):
+    """A checkpoint whose probe records do not fit in device memory is refused;
+    the job, whose fields are in the second set, goes on with its own."""
+    spec, _ = problems.config_2d_tmz(precision=abi.F32, n=192, ncyl=2, nfreq=8, npml=16)
+    spec.add_probe((96, 96, 0), (abi.EZ,))
+    A = gpu.Job(spec, tile=4)
+    A.step(1, 1500)  # more probe records than a new job's buffer holds
+    long = A.save_state()
+    A.close()
+    J = gpu.Job(spec, tile=4)
+    J.step(1, 8)
+    rng = np.random.default_rng(1).standard_normal((1, 192, 192))
+    rng[:, :16] = rng[:, -16:] = rng[:, :, :16] = rng[:, :, -16:] = 0
+    J.set_field(abi.EZ, rng)
+    J.step(9, 8)  # one launch: the current fields are in the second set
+    K = gpu.Job(spec, tile=4)
+    K.load_state(J.save_state())
+    J.step(17, 8)
+    K.step(17, 8)
+    try:
+        gpu.fail_alloc_after(0)
+        with pytest.raises(gpu.FdtdError) as e:
+            J.load_state(long)
+        assert e.value.code == abi.FDTD_ENOMEM
+    finally:
+        gpu.fail_alloc_after(-1)
+    J.step(25, 40)
+    K.step(25, 40)
+    for a, b in zip(state_of(J, FIELDS_TM), state_of(K, FIELDS_TM)):
+        np.testing.assert_array_equal(a, b)
+    assert np.any(J.get_field(abi.EZ))
+    J.close()
+    K.close()
