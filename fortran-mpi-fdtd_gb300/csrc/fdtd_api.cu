@@ -208,6 +208,13 @@ struct fdtd_job {
   // 1D per-launch source values
   double *d_srcval = nullptr;
   long long srcval_cap = 0;
+  // the host's copies of the last calls' 1D source values, each with the event
+  // after which no copy to the device reads it any more
+  struct SrcCall {
+    std::vector<double> v;
+    cudaEvent_t done = nullptr;
+  } src_call[4];
+  unsigned src_next = 0;
   // 2D/3D: amp*g(t) of every step, [(n-1)*nsrc + q], on the device
   std::vector<double> srctab;
   double *d_srctab = nullptr;
@@ -248,6 +255,7 @@ struct fdtd_job {
   Block3 b3{};
   void *spb3[6] = {};
   size_t b3_bytes[6] = {};  // of the flags, slot map, first step's dispersive state, its sampled rows, order, segments
+  std::vector<std::vector<char>> put_host;  // during commit: host data of queued copies
   std::vector<int> ade_cell_host;      // during commit: the dispersive cells and their ids
   std::vector<uint8_t> ade_mat_host;
   FusedMaps fmaps[2]{};
@@ -370,17 +378,30 @@ int alloc_state(fdtd_job *J, void **p, size_t bytes, int esz = 0) {
   return FDTD_OK;
 }
 
-// Host data go to the device on the job's stream: a plain cudaMemcpy from
-// pageable memory may return before its last bytes have landed, and the job's
-// streams, which do not wait for the legacy stream, could then run ahead of it
-// (seen on a busy GPU: a source table read before it was there).  The copy has
-// left the host buffer when the call returns.
+// Host data to the device.  The copy is on the job's stream: a plain cudaMemcpy
+// from pageable memory may return before its last bytes have landed, and the
+// job's streams, which do not wait for the legacy stream, could then run ahead
+// of it (seen on a busy GPU: a source table read before it was there).  A queued
+// copy may still read a host buffer that goes away, so it is waited for; of the
+// small tables of set-up the job keeps copies until its commit has waited once
+// (a wait each: 0.1-0.2 ms of a commit of 0.8).
+int put_dev(fdtd_job *J, void *dst, const void *src, size_t bytes) {
+  const bool keep = !J->committed && bytes <= 32768;
+  if (keep) {
+    J->put_host.emplace_back((const char *)src, (const char *)src + bytes);
+    src = J->put_host.back().data();
+  }
+  CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, J->stream));
+  if (!keep) CK(cudaStreamSynchronize(J->stream));
+  return FDTD_OK;
+}
+
 template <typename T>
 int upload_vec(fdtd_job *J, void **dst, const std::vector<double> &v) {
   std::vector<T> t(v.begin(), v.end());
   int rc = alloc_dev(J, dst, t.size() * sizeof(T));
   if (rc) return rc;
-  CK(cudaMemcpyAsync(*dst, t.data(), t.size() * sizeof(T), cudaMemcpyHostToDevice, J->stream));
+  if ((rc = put_dev(J, *dst, t.data(), t.size() * sizeof(T)))) return rc;
   J->h2d += t.size() * sizeof(T);
   return FDTD_OK;
 }
@@ -555,7 +576,7 @@ int split_2d(fdtd_job *J, const std::vector<uint8_t> &rf) {
   int rc;
   if (!edge.empty()) {
     if ((rc = alloc_dev(J, (void **)&J->d_edge, edge.size() * sizeof(int)))) return rc;
-    CK(cudaMemcpyAsync(J->d_edge, edge.data(), edge.size() * sizeof(int), cudaMemcpyHostToDevice, J->stream));
+    if ((rc = put_dev(J, J->d_edge, edge.data(), edge.size() * sizeof(int)))) return rc;
     J->h2d += edge.size() * sizeof(int);
   }
   return make_branches(J);
@@ -596,7 +617,7 @@ int split_3d(fdtd_job *J, const std::vector<uint8_t> &rf) {
   int rc;
   if (!edge.empty()) {
     if ((rc = alloc_dev(J, (void **)&J->d_edge, edge.size() * sizeof(int)))) return rc;
-    CK(cudaMemcpyAsync(J->d_edge, edge.data(), edge.size() * sizeof(int), cudaMemcpyHostToDevice, J->stream));
+    if ((rc = put_dev(J, J->d_edge, edge.data(), edge.size() * sizeof(int)))) return rc;
     J->h2d += edge.size() * sizeof(int);
   }
   return make_branches(J);
@@ -984,10 +1005,10 @@ int commit_impl(fdtd_job *J) {
       }
   }
   if ((rc = alloc_dev(J, (void **)&J->d_mat, (size_t)N))) return rc;
-  CK(cudaMemcpyAsync(J->d_mat, mat.data(), (size_t)N, cudaMemcpyHostToDevice, J->stream));
+  if ((rc = put_dev(J, J->d_mat, mat.data(), (size_t)N))) return rc;
   J->h2d += (uint64_t)N;
   if ((rc = alloc_dev(J, &J->d_mc, sizeof(MatCoef<T>) * kMaxMat))) return rc;
-  CK(cudaMemcpyAsync(J->d_mc, mc.data(), sizeof(MatCoef<T>) * kMaxMat, cudaMemcpyHostToDevice, J->stream));
+  if ((rc = put_dev(J, J->d_mc, mc.data(), sizeof(MatCoef<T>) * kMaxMat))) return rc;
   J->h2d += sizeof(MatCoef<T>) * kMaxMat + sizeof(AdeCoef<T>) * ac.size();
   {
     std::vector<double> ca(kMaxMat, 0.0), cs(kMaxMat, 0.0);
@@ -998,7 +1019,7 @@ int commit_impl(fdtd_job *J) {
     if ((rc = upload_vec<T>(J, &J->d_mcs, cs))) return rc;
   }
   if ((rc = alloc_dev(J, &J->d_ac, sizeof(AdeCoef<T>) * std::max<size_t>(1, ac.size())))) return rc;
-  if (!ac.empty()) CK(cudaMemcpyAsync(J->d_ac, ac.data(), sizeof(AdeCoef<T>) * ac.size(), cudaMemcpyHostToDevice, J->stream));
+  if (!ac.empty() && (rc = put_dev(J, J->d_ac, ac.data(), sizeof(AdeCoef<T>) * ac.size()))) return rc;
   J->ac_host.assign((const char *)ac.data(), (const char *)ac.data() + sizeof(AdeCoef<T>) * ac.size());
   J->ade_kind = ac.empty() ? -1 : ac[0].kind;  // the device update all the dispersive materials share, or -1
   for (const AdeCoef<T> &a : ac)
@@ -1028,8 +1049,8 @@ int commit_impl(fdtd_job *J) {
   if ((rc = alloc_dev(J, (void **)&J->d_ade_cell, sizeof(int) * std::max(1, J->nade)))) return rc;
   if ((rc = alloc_dev(J, (void **)&J->d_ade_mat, std::max(1, J->nade)))) return rc;
   if (J->nade) {
-    CK(cudaMemcpyAsync(J->d_ade_cell, ade_cell.data(), sizeof(int) * J->nade, cudaMemcpyHostToDevice, J->stream));
-    CK(cudaMemcpyAsync(J->d_ade_mat, ade_mat.data(), J->nade, cudaMemcpyHostToDevice, J->stream));
+    if ((rc = put_dev(J, J->d_ade_cell, ade_cell.data(), sizeof(int) * J->nade))) return rc;
+    if ((rc = put_dev(J, J->d_ade_mat, ade_mat.data(), J->nade))) return rc;
     J->h2d += (uint64_t)J->nade * (sizeof(int) + 1);
   }
   J->ade_nf = 0;
@@ -1191,7 +1212,7 @@ int commit_impl(fdtd_job *J) {
       for (int j = 0; j < ny; ++j)
         if (j < J->slab_rows || j >= ny - J->slab_rows) rf[j] |= ROW_SLAB;
     if ((rc = alloc_dev(J, (void **)&J->d_rowflag, (size_t)ny))) return rc;
-    CK(cudaMemcpyAsync(J->d_rowflag, rf.data(), (size_t)ny, cudaMemcpyHostToDevice, J->stream));
+    if ((rc = put_dev(J, J->d_rowflag, rf.data(), (size_t)ny))) return rc;
     J->h2d += (uint64_t)ny;
     if ((rc = split_2d(J, rf))) return rc;
   } else if (J->dim == 3) {
@@ -1203,7 +1224,7 @@ int commit_impl(fdtd_job *J) {
           rf[(size_t)k * ny + j] |= ROW_SRC;
     }
     if ((rc = alloc_dev(J, (void **)&J->d_rowflag, rf.size()))) return rc;
-    CK(cudaMemcpyAsync(J->d_rowflag, rf.data(), rf.size(), cudaMemcpyHostToDevice, J->stream));
+    if ((rc = put_dev(J, J->d_rowflag, rf.data(), rf.size()))) return rc;
     J->h2d += rf.size();
     if ((rc = split_3d(J, rf))) return rc;
   }
@@ -1225,7 +1246,7 @@ int commit_impl(fdtd_job *J) {
       }
     }
     if ((rc = alloc_dev(J, (void **)&J->d_uni, bits.size() * sizeof(uint32_t)))) return rc;
-    CK(cudaMemcpyAsync(J->d_uni, bits.data(), bits.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, J->stream));
+    if ((rc = put_dev(J, J->d_uni, bits.data(), bits.size() * sizeof(uint32_t)))) return rc;
     J->h2d += bits.size() * sizeof(uint32_t);
     J->uni_words = words;
   }
@@ -1233,7 +1254,7 @@ int commit_impl(fdtd_job *J) {
   J->acc_total = acc;
   if (!omega.empty()) {
     if ((rc = alloc_dev(J, (void **)&J->d_omega, omega.size() * sizeof(double)))) return rc;
-    CK(cudaMemcpyAsync(J->d_omega, omega.data(), omega.size() * sizeof(double), cudaMemcpyHostToDevice, J->stream));
+    if ((rc = put_dev(J, J->d_omega, omega.data(), omega.size() * sizeof(double)))) return rc;
     // e^{i w s dt} for the slots of a DFT ring
     std::vector<double> rot(omega.size() * 2 * kStageSteps);
     for (size_t f = 0; f < omega.size(); ++f)
@@ -1243,7 +1264,7 @@ int commit_impl(fdtd_job *J) {
         rot[(f * kStageSteps + sl) * 2 + 1] = std::sin(ph);
       }
     if ((rc = alloc_dev(J, (void **)&J->d_rot, rot.size() * sizeof(double)))) return rc;
-    CK(cudaMemcpyAsync(J->d_rot, rot.data(), rot.size() * sizeof(double), cudaMemcpyHostToDevice, J->stream));
+    if ((rc = put_dev(J, J->d_rot, rot.data(), rot.size() * sizeof(double)))) return rc;
     J->h2d += rot.size() * sizeof(double);
     J->h2d += omega.size() * sizeof(double);
   }
@@ -1265,6 +1286,8 @@ int commit_impl(fdtd_job *J) {
   if (J->fused_ok && J->tile != fused_tile(J) && !J->block3_ok) free_fused(J);
   std::vector<int>().swap(J->ade_cell_host);
   std::vector<uint8_t>().swap(J->ade_mat_host);
+  CK(cudaStreamSynchronize(J->stream));
+  J->put_host.clear();
   if ((rc = kernel_flag(J))) return rc;
   J->committed = true;
   return FDTD_OK;
@@ -1356,7 +1379,7 @@ int setup_line(fdtd_job *J) {
     std::vector<int> slot((size_t)N, -1);
     for (int q = 0; q < J->nade; ++q) slot[J->ade_cell_host[q]] = q;
     if ((rc = alloc_dev(J, (void **)&J->d_line_slot, N * sizeof(int)))) return rc;
-    CK(cudaMemcpyAsync(J->d_line_slot, slot.data(), N * sizeof(int), cudaMemcpyHostToDevice, J->stream));
+    if ((rc = put_dev(J, J->d_line_slot, slot.data(), N * sizeof(int)))) return rc;
     J->h2d += N * sizeof(int);
     if ((rc = alloc_dev(J, &J->ade_b, ade_bytes(J)))) return rc;
   }
@@ -1471,7 +1494,7 @@ int setup_block(fdtd_job *J) {
     *dst = nullptr;
     B.bytes[q] = bytes;
     if (const int e = alloc_dev(J, dst, bytes)) return e;
-    if (src) CK(cudaMemcpyAsync(*dst, src, bytes, cudaMemcpyHostToDevice, J->stream));
+    if (src && (rc = put_dev(J, *dst, src, bytes))) return rc;
     J->h2d += src ? bytes : 0;
     return FDTD_OK;
   };
@@ -1666,8 +1689,7 @@ int setup_block3(fdtd_job *J) {
   });
   J->b3_bytes[4] = (size_t)nt * sizeof(int);
   if ((rc = alloc_dev(J, (void **)&b.order, J->b3_bytes[4]))) return rc;
-  CK(cudaMemcpyAsync((void *)b.order, order.data(), J->b3_bytes[4], cudaMemcpyHostToDevice, J->stream));
-  CK(cudaStreamSynchronize(J->stream));
+  if ((rc = put_dev(J, (void *)b.order, order.data(), J->b3_bytes[4]))) return rc;
   J->h2d += J->b3_bytes[4];
   if (J->nade > 0) {
     b.one_gold = J->ac_host.size() == sizeof(AdeCoef<float>) && ac[0].kind == MK_GOLD;
@@ -1688,12 +1710,11 @@ int setup_block3(fdtd_job *J) {
     }
     J->b3_bytes[1] = slot.size() * sizeof(int);
     if ((rc = alloc_dev(J, (void **)&b.slot, J->b3_bytes[1]))) return rc;
-    CK(cudaMemcpyAsync((void *)b.slot, slot.data(), J->b3_bytes[1], cudaMemcpyHostToDevice, J->stream));
+    if ((rc = put_dev(J, (void *)b.slot, slot.data(), J->b3_bytes[1]))) return rc;
     J->h2d += J->b3_bytes[1];
     J->b3_bytes[2] = ade_bytes(J);
     if ((rc = alloc_dev(J, (void **)&b.ade_mid, J->b3_bytes[2]))) return rc;
     if (!J->ade_b && (rc = alloc_dev(J, &J->ade_b, ade_bytes(J)))) return rc;
-    CK(cudaStreamSynchronize(J->stream));
   }
   // the rows with samples, numbered
   std::vector<int> seg(rows, 0);
@@ -1705,10 +1726,9 @@ int setup_block3(fdtd_job *J) {
     if ((rc = alloc_dev(J, (void **)&b.first, J->b3_bytes[3]))) return rc;
     J->b3_bytes[5] = rows * sizeof(int);
     if ((rc = alloc_dev(J, (void **)&b.seg, J->b3_bytes[5]))) return rc;
-    CK(cudaMemcpyAsync((void *)b.seg, seg.data(), J->b3_bytes[5], cudaMemcpyHostToDevice, J->stream));
+    if ((rc = put_dev(J, (void *)b.seg, seg.data(), J->b3_bytes[5]))) return rc;
     J->h2d += J->b3_bytes[5];
   }
-  CK(cudaStreamSynchronize(J->stream));
   J->block3_ok = true;
   return FDTD_OK;
 }
@@ -1924,12 +1944,9 @@ int ensure_srctab(fdtd_job *J, int n_max) {
     J->srctab_cap_steps = cap;
     J->dev_bytes += (uint64_t)cap * nsrc * sizeof(double);
     destroy_graph(J);  // the captured launches hold the old pointer
-    CK(cudaMemcpyAsync(J->d_srctab, J->srctab.data(), (size_t)n_max * nsrc * sizeof(double), cudaMemcpyHostToDevice, J->stream));
-  } else {
-    CK(cudaMemcpyAsync(J->d_srctab + (size_t)old_steps * nsrc, J->srctab.data() + (size_t)old_steps * nsrc,
-                       (size_t)(n_max - old_steps) * nsrc * sizeof(double), cudaMemcpyHostToDevice, J->stream));
-    CK(cudaStreamSynchronize(J->stream));  // the host vector may grow again
   }
+  const size_t at = nb ? 0 : (size_t)old_steps * nsrc;  // a new table takes all of it
+  if (const int rc = put_dev(J, J->d_srctab + at, J->srctab.data() + at, ((size_t)n_max * nsrc - at) * sizeof(double))) return rc;
   J->h2d += (uint64_t)(n_max - old_steps) * nsrc * sizeof(double);
   return FDTD_OK;
 }
@@ -2773,10 +2790,19 @@ int line_run(fdtd_job *J, int n_first, int n_steps, int stages) {
     J->srcval_cap = cap;
     J->dev_bytes += cap * sizeof(double);
   }
-  // the sources' values of steps st0..st1-1 of the call, to the device
+  // The sources' values of steps st0..st1-1 of the call, to the device.  They
+  // are queued from a buffer of the job, so that the host goes on: the calls take
+  // four in turn, and wait for the copies of the fourth call before.
+  fdtd_job::SrcCall &sc = J->src_call[J->src_next % 4];
+  if (p.nsrc) {
+    ++J->src_next;
+    if (!sc.done) CK(cudaEventCreateWithFlags(&sc.done, cudaEventDisableTiming));
+    else CK(cudaEventSynchronize(sc.done));
+    sc.v.resize((size_t)n_steps * p.nsrc);
+  }
   auto sources = [&](int st0, int st1) -> int {
     if (!p.nsrc || st1 <= st0) return FDTD_OK;
-    std::vector<double> v((size_t)(st1 - st0) * p.nsrc);
+    double *const v = sc.v.data() + (size_t)st0 * p.nsrc;
     for (int st = st0; st < st1; ++st) {
       const double t = (double)(n_first + st - 1) * J->g.dt;
       int q = 0;
@@ -2786,8 +2812,9 @@ int line_run(fdtd_job *J, int n_first, int n_steps, int stages) {
         ++q;
       }
     }
-    CK(cudaMemcpyAsync(J->d_srcval + (size_t)st0 * p.nsrc, v.data(), v.size() * sizeof(double), cudaMemcpyHostToDevice,
-                       J->stream));  // pageable: v has been read when the call returns
+    CK(cudaMemcpyAsync(J->d_srcval + (size_t)st0 * p.nsrc, v, (size_t)(st1 - st0) * p.nsrc * sizeof(double),
+                       cudaMemcpyHostToDevice, J->stream));
+    CK(cudaEventRecord(sc.done, J->stream));
     return FDTD_OK;
   };
   p.srcval = J->d_srcval;
@@ -3303,6 +3330,8 @@ int fdtd_destroy(fdtd_job *J) {
     if (J->ev_prog[q]) cudaEventDestroy(J->ev_prog[q]);
   }
   if (J->ev_fork) cudaEventDestroy(J->ev_fork);
+  for (auto &c : J->src_call)
+    if (c.done) cudaEventDestroy(c.done);
   if (J->fold_stream) cudaStreamDestroy(J->fold_stream);
   if (J->ev_ffork) cudaEventDestroy(J->ev_ffork);
   if (J->ev_fjoin) cudaEventDestroy(J->ev_fjoin);
