@@ -2214,8 +2214,8 @@ int tune_tiles(fdtd_job *J) {
     J->tile = 1;
     return FDTD_OK;
   }
-  if (off && off[0] == 'b' && J->block3_ok) {  // "block": the 3D block-step kernel where it is offered
-    J->tile = kBlock3Tile;
+  if (off && off[0] == 'b' && (J->dim == 2 ? J->fused_ok : J->block3_ok)) {  // "block": a block-step kernel where one is offered
+    J->tile = J->dim == 2 ? fused_tile(J) : kBlock3Tile;
     return FDTD_OK;
   }
   int lg = 0;

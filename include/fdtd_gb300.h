@@ -472,8 +472,9 @@ int fdtd_kernel_time(fdtd_job *job, int32_t kind, int64_t *launches, double *ms)
  * the whole grid per launch; FP32, 4-cell vectors, periodic or not, no
  * reference slabs or TFSF box; second copies of the six fields, the stored
  * PML parts and the dispersive state, and none if the device has no room for
- * them); it cannot be pinned, but environment FDTD_TUNE=block takes it
- * wherever it is offered.  Results do not depend on the shape.  Environment
+ * them); it cannot be pinned.  Environment FDTD_TUNE=block takes the 2D and
+ * 3D block-step kernels wherever they are offered, without timing.  Results do
+ * not depend on the shape.  Environment
  * FDTD_NO_TMA leaves the TMA-staged kernels out, FDTD_NO_FUSED the fused and
  * block-step ones.  fdtd_get_tile returns the shape in use (0: the job has no
  * core kernels; 10: the 3D block-step kernel). */

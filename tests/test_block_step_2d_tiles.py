@@ -1,0 +1,34 @@
+"""Both tile shapes of the 2D block-step kernel against the half-step kernels, bit
+for bit, with the kernel chosen by environment, so that no timing decides what
+is compared: the tall shape (taken once its tiles outnumber the SMs) with odd
+rows, periodic axes, several materials, many sampled rows and tiles whose
+dispersive state goes past shared memory; the low shape where it cannot be
+pinned."""
+import numpy as np
+import pytest
+
+from fdtd_gpu import abi
+from test_block_step_2d import BLOCK, gpu, make, result  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("te", [False, True])
+@pytest.mark.parametrize("nx,ny,kw", [
+    # 112 x 48 cells owned: 13 x 14 tiles and more
+    (1344, 672, {}), (1345, 673, dict(sub=True, lorentz=True)), (1347, 625, dict(vertical=True, lorentz=True)),
+    (1348, 630, dict(per=(1, 0), sub=True)), (1401, 671, dict(pml=0, per=(1, 1), lorentz=True)),
+    (1920, 1200, dict(sub=True, vertical=True)),
+    # 112 x 16 cells owned
+    (227, 81, dict(vertical=True, lorentz=True)), (231, 90, dict(pml=0, per=(1, 1), vertical=True)),
+])
+def test_block_step_equals_half_steps(gpu, monkeypatch, te, nx, ny, kw):  # noqa: F811
+    monkeypatch.setenv("FDTD_TUNE", "block")
+    spec = make(nx, ny, te, **kw)
+    calls = (1, 2, 5, 8, 9, 64, 31)
+    used, got = result(gpu, spec, calls)
+    assert used == BLOCK
+    split, ref = result(gpu, spec, (sum(calls),), tile=2)
+    assert split == 2 and any(np.any(r) for r in ref)
+    for a, b in zip(got, ref):
+        np.testing.assert_array_equal(a, b)
