@@ -315,10 +315,18 @@ void keep_pool_memory(int dev) {
 // before one fails (-1: none fails)
 std::atomic<long long> g_fail_after{-1};
 
+// fdtd_debug_fail_launch: the same for launches of the multi-step kernels
+std::atomic<long long> g_fail_launch{-1};
+
+// whether a failure counted down by g is due now
+bool fails_now(std::atomic<long long> &g) {
+  long long left = g.load();
+  while (left >= 0 && !g.compare_exchange_weak(left, left - 1)) {}
+  return left == 0;
+}
+
 cudaError_t pool_alloc(fdtd_job *J, void **p, size_t bytes) {
-  long long left = g_fail_after.load();
-  while (left >= 0 && !g_fail_after.compare_exchange_weak(left, left - 1)) {}
-  if (left == 0) {
+  if (fails_now(g_fail_after)) {
     *p = nullptr;
     return cudaErrorMemoryAllocation;
   }
@@ -2164,16 +2172,18 @@ void block3_buffers(const fdtd_job *J, StepParams<float> &p, Block3 &b, int from
 // stream.  Returns the kernels launched, -1 on failure.
 int launch_blocks(fdtd_job *J, const StepParams<float> &p, const BlockPlan &pl) {
   const bool both = pl.ngen > 0 && pl.ngen < pl.ntiles && !J->prof;
-  if (!both) return launch_step2d_block(p, pl, true, J->stream) + launch_step2d_block(p, pl, false, J->stream);
-  auto ok = [](cudaError_t e) {
-    if (e != cudaSuccess) set_err(FDTD_ECUDA, "block-step launch: %s", cudaGetErrorString(e));
-    return e == cudaSuccess;
-  };
-  if (!ok(cudaEventRecord(J->ev_fork, J->stream)) || !ok(cudaStreamWaitEvent(J->side[0], J->ev_fork, 0))) return -1;
-  int n = launch_step2d_block(p, pl, true, J->stream);
-  n += launch_step2d_block(p, pl, false, J->side[0]);
-  if (!ok(cudaEventRecord(J->ev_join[0], J->side[0])) || !ok(cudaStreamWaitEvent(J->stream, J->ev_join[0], 0))) return -1;
-  return n;
+  cudaStream_t side = both ? J->side[0] : J->stream;
+  cudaError_t e = fails_now(g_fail_launch) ? cudaErrorLaunchFailure : cudaSuccess;
+  if (both && e == cudaSuccess && (e = cudaEventRecord(J->ev_fork, J->stream)) == cudaSuccess)
+    e = cudaStreamWaitEvent(side, J->ev_fork, 0);
+  const int n0 = e == cudaSuccess ? launch_step2d_block(p, pl, true, J->stream) : -1;
+  const int n1 = n0 >= 0 ? launch_step2d_block(p, pl, false, side) : -1;
+  if (both && n1 >= 0 && (e = cudaEventRecord(J->ev_join[0], side)) == cudaSuccess) e = cudaStreamWaitEvent(J->stream, J->ev_join[0], 0);
+  if (n1 < 0 || e != cudaSuccess) {
+    set_err(FDTD_ECUDA, "2D block-step launch: %s", cudaGetErrorString(e != cudaSuccess ? e : cudaGetLastError()));
+    return -1;
+  }
+  return n0 + n1;
 }
 
 // The same in 3D: the tiles with dispersive cells beside the others, which run
@@ -2181,8 +2191,9 @@ int launch_blocks(fdtd_job *J, const StepParams<float> &p, const BlockPlan &pl) 
 int launch_blocks3(fdtd_job *J, const StepParams<float> &p, const Block3 &b, int k) {
   const bool both = b.nade > 0 && b.nade < b.ntx * b.nty * b.ntz && !J->prof;
   cudaStream_t side = both ? J->side[0] : J->stream;
-  cudaError_t e = cudaSuccess;
-  if (both && (e = cudaEventRecord(J->ev_fork, J->stream)) == cudaSuccess) e = cudaStreamWaitEvent(side, J->ev_fork, 0);
+  cudaError_t e = fails_now(g_fail_launch) ? cudaErrorLaunchFailure : cudaSuccess;
+  if (both && e == cudaSuccess && (e = cudaEventRecord(J->ev_fork, J->stream)) == cudaSuccess)
+    e = cudaStreamWaitEvent(side, J->ev_fork, 0);
   const int n0 = e == cudaSuccess ? launch_step3d_block(p, b, k, true, J->stream) : -1;
   const int n1 = n0 >= 0 ? launch_step3d_block(p, b, k, false, side) : -1;
   if (both && n1 >= 0 && (e = cudaEventRecord(J->ev_join[0], side)) == cudaSuccess) e = cudaStreamWaitEvent(J->stream, J->ev_join[0], 0);
@@ -2279,19 +2290,20 @@ int tune_tiles(fdtd_job *J) {
     run_parts<T>(J, p, parts, false, true);
   };
   int from = 0;
+  bool failed = false;  // a launch of the block-step kernels
   auto cores = [&](int c) {
     if constexpr (sizeof(T) == 4) {
       if (J->dim == 2 && c == fused_tile(J)) {
         StepParams<float> q = p;
         block_buffers(J, q, pl, 0);
-        launch_blocks(J, q, pl);
+        failed |= launch_blocks(J, q, pl) < 0;
         return;
       }
       if (J->dim == 3 && c == kBlock3Tile) {
         StepParams<float> q = p;
         Block3 b3;
         block3_buffers(J, q, b3, from ^= 1);  // to and fro, as steps run
-        launch_blocks3(J, q, b3, 2);
+        failed |= launch_blocks3(J, q, b3, 2) < 0;
         return;
       }
       if (J->dim == 3 && c == fused_tile(J)) {
@@ -2323,6 +2335,10 @@ int tune_tiles(fdtd_job *J) {
     float ms = time5([&] { cores(c); }) / (block ? (float)(J->dim == 2 ? pl.ks : 2) : 1.f);  // of a step
     // (the first runs of the 3D block-step kernel take a quarter longer than all later ones)
     if (J->dim == 3 && block) ms = std::min(ms, time5([&] { cores(c); }) / 2.f);
+    if (block && failed) {  // a kernel that did not run is no candidate
+      cudaGetLastError();
+      continue;
+    }
     if (J->dim == 3 && c < fused_tile(J) && ms < best_split) {
       best_split = ms;
       J->split_tile = c;
@@ -2336,6 +2352,7 @@ int tune_tiles(fdtd_job *J) {
   cudaEventDestroy(b);
   CK(cudaGetLastError());
   J->tile = choice;
+  if (failed) return FDTD_OK;  // the next job of the kind tries again
   std::lock_guard<std::mutex> lk(g_tune_mu);
   g_tune[key] = choice | J->split_tile << 8;
   return FDTD_OK;
@@ -2431,9 +2448,9 @@ int block_step(fdtd_job *J, int n, int k, int slot, bool graph) {
   if (!graph) ev_record(J, FDTD_KERNEL_STEP, false);
   if (ran < 0) return FDTD_ECUDA;
   J->launches += ran;
-  J->pp ^= 1;
   J->prog_prev = -1;
   CK(cudaGetLastError());
+  J->pp ^= 1;
   return FDTD_OK;
 }
 
@@ -2462,9 +2479,9 @@ int block3_step(fdtd_job *J, int n, int k, int slot, bool graph) {
   p.n = n + k - 1;
   p.ex = p.exo; p.ey = p.eyo; p.ez = p.ezo; p.hx = p.hxo; p.hy = p.hyo; p.hz = p.hzo;
   J->launches += launch_gather<float>(p, J->stream);
-  J->pp ^= 1;
   J->prog_prev = -1;
   CK(cudaGetLastError());
+  J->pp ^= 1;
   return FDTD_OK;
 }
 
@@ -2480,6 +2497,7 @@ int fused_step(fdtd_job *J, int n, int slot, bool graph) {
     (void)n; (void)slot; (void)graph;
     return set_err(FDTD_ESTATE, "the fused step kernel is FP32 only");
   } else {
+    if (fails_now(g_fail_launch)) return set_err(FDTD_ECUDA, "fused step launch: %s", cudaGetErrorString(cudaErrorLaunchFailure));
     const int from = J->pp, to = 1 - from;
     float *A[6], *B[6];
     for (int c = 0; c < 6; ++c) {
@@ -2514,9 +2532,9 @@ int fused_step(fdtd_job *J, int n, int slot, bool graph) {
     g.slot = slot;
     ring_params(J, g, graph);
     J->launches += launch_gather<float>(g, J->stream);
-    J->pp = to;
     J->prog_prev = -1;
     CK(cudaGetLastError());
+    J->pp = to;
     return FDTD_OK;
   }
 }
@@ -2720,8 +2738,8 @@ int line_blocks(fdtd_job *J, LineParams<T> p, T *stage, F sources) {
         b.pexo[l][s] = out.pex[l][s];
         b.phzo[l][s] = out.phz[l][s];
       }
-    const int ran = launch_line1d_block<T>(q[from], b, V, J->stream);
-    if (!ran) return set_err(FDTD_ECUDA, "1D block-step launch: %s", cudaGetErrorString(cudaGetLastError()));
+    const int ran = fails_now(g_fail_launch) ? -1 : launch_line1d_block<T>(q[from], b, V, J->stream);
+    if (ran < 0) return set_err(FDTD_ECUDA, "1D block-step launch: %s", cudaGetErrorString(cudaGetLastError()));
     J->launches += ran;
     s0 += b.ks;
   }
@@ -3606,6 +3624,11 @@ int fdtd_debug_wait_limit(fdtd_job *J, int32_t rounds) {
   if (!J) return set_err(FDTD_EINVAL, "null job");
   J->wait_limit = rounds < 0 ? kWaitLimit : (unsigned)rounds;
   destroy_graph(J);  // the captured launches hold the old limit
+  return FDTD_OK;
+}
+
+int fdtd_debug_fail_launch(int32_t after) {
+  g_fail_launch.store(after < 0 ? -1 : after);
   return FDTD_OK;
 }
 

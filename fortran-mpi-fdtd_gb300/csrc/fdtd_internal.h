@@ -318,7 +318,7 @@ BlockShape block_shape(int shape);
 // bytes of dynamic shared memory (and the plan's offsets) for tiles with at
 // most max_ade dispersive cells; sets cap
 void block_smem(BlockPlan &pl, int layout, int max_ade, bool split, bool smp_rows);
-// the general or the plain tiles of a launch; returns the kernels launched
+// the general or the plain tiles of a launch; returns the kernels launched, -1 on failure
 int launch_step2d_block(const StepParams<float> &p, const BlockPlan &pl, bool gen, void *stream);
 void launch_tile_flags(const uint8_t *mat, const uint8_t *rowflag, const Tile2 *tiles, int ntiles, int R, int NW, int V,
                        const BlockGeom &g, uint16_t *out, void *stream);
@@ -468,7 +468,7 @@ struct LineBlock {
   int s0, ks, own;             // first step of this launch (from p.n_first), its steps, cells per block
 };
 // V: cells per thread (1 or 2; a block holds 128 V cells, own + 2 ks of them);
-// returns the kernels launched
+// returns the kernels launched, -1 on failure
 template <typename T> int launch_line1d_block(const LineParams<T> &p, const LineBlock<T> &b, int V, void *stream);
 template <typename T> void launch_line1d_stage(const LineParams<T> &p, T *stage, long long stage_row, void *stream);
 

@@ -426,8 +426,8 @@ __global__ void __launch_bounds__(32 * kLineWarps) line1d_block(const __grid_con
 template <typename T, int V, bool INC, int KIND>
 int launch_v(const LineParams<T> &p, const LineBlock<T> &b, cudaStream_t s) {
   auto kern = line1d_block<T, V, INC, KIND>;
-  static const cudaError_t attr = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-  if (attr != cudaSuccess) return 0;
+  static std::atomic<unsigned long long> done{0};
+  if (!smem_limit(kern, 96 * 1024, done)) return -1;
   const size_t sm = (size_t)(kLineSteps * (kMaxSrc + kLineRecords * 4) + (KIND == -1 ? (2 + p.ade_nf) * 32 * kLineWarps * V : 0)) * sizeof(T);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((p.N + b.own - 1) / b.own);
@@ -439,7 +439,7 @@ int launch_v(const LineParams<T> &p, const LineBlock<T> &b, cudaStream_t s) {
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, p, b) == cudaSuccess ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, p, b) == cudaSuccess ? 1 : -1;
 }
 
 template <typename T, int V, bool INC>

@@ -779,8 +779,8 @@ int launch_block_k(const StepParams<T> &p, const BlockPlan &pl, cudaStream_t s) 
   constexpr int R = GEN ? Shapes::RB[S] : Shapes::RA[S], NW = GEN ? Shapes::NB[S] : Shapes::NA[S];
   constexpr int V = Shapes::V;
   auto kern = step2d_block<L, V, R, NW, GEN ? 1 : 2, KIND, GEN>;
-  static const cudaError_t attr = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-  if (attr != cudaSuccess) return 0;
+  static std::atomic<unsigned long long> done{0};
+  if (!smem_limit(kern, 227 * 1024, done)) return -1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(GEN ? pl.ngen : pl.ntiles - pl.ngen);
   cfg.blockDim = dim3(32 * NW);
@@ -791,8 +791,7 @@ int launch_block_k(const StepParams<T> &p, const BlockPlan &pl, cudaStream_t s) 
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kern, p, pl);
-  return 1;
+  return cudaLaunchKernelEx(&cfg, kern, p, pl) == cudaSuccess ? 1 : -1;
 }
 
 template <int L, int S>

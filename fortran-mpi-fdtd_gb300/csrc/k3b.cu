@@ -712,9 +712,8 @@ int launch3b(const StepParams<float> &p, const Block3 &b, cudaStream_t s) {
   const int blocks = ADE ? b.nade : b.ntx * b.nty * b.ntz - b.nade;
   if (blocks == 0) return 0;
   const int smem = 42 * 32 * kB3Warps * (int)sizeof(f2);
-  static const bool attr =
-      cudaFuncSetAttribute(step3d_block<NS, kB3Warps, ADE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess;
-  if (!attr) return -1;
+  static std::atomic<unsigned long long> done{0};
+  if (!smem_limit(step3d_block<NS, kB3Warps, ADE>, smem, done)) return -1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(blocks);
   cfg.blockDim = dim3(32 * kB3Warps);

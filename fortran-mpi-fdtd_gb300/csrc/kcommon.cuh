@@ -2,6 +2,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <atomic>
+
 #include "fdtd_internal.h"
 
 namespace fdtd {
@@ -35,6 +37,19 @@ __device__ __forceinline__ float fma1(float a, float b, float c) { return __fmaf
 __device__ __forceinline__ double fma1(double a, double b, double c) { return __fma_rn(a, b, c); }
 __device__ __forceinline__ float mul1(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ double mul1(double a, double b) { return __dmul_rn(a, b); }
+
+// A kernel's limit of dynamic shared memory, once on each device (bits of
+// `done`); false: it could not be set, and the next launch tries again.
+template <typename K>
+bool smem_limit(K kern, int bytes, std::atomic<unsigned long long> &done) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  const unsigned long long bit = dev < 64 ? 1ull << dev : 0;
+  if (done.load() & bit) return true;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return false;
+  done.fetch_or(bit);
+  return true;
+}
 
 // launch a step kernel with a programmatic dependency on the kernel before it
 // on the stream (the kernel starts with pdl_wait).  With `ev`, the launch also

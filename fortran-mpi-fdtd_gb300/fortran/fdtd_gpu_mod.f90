@@ -313,6 +313,10 @@ module fdtd_gpu_mod
        import :: c_int, c_int32_t
        integer(c_int32_t), value :: after
      end function fdtd_debug_fail_alloc
+     integer(c_int) function fdtd_debug_fail_launch(after) bind(c, name='fdtd_debug_fail_launch')
+       import :: c_int, c_int32_t
+       integer(c_int32_t), value :: after
+     end function fdtd_debug_fail_launch
      integer(c_int) function fdtd_debug_wait_limit(job, rounds) bind(c, name='fdtd_debug_wait_limit')
        import :: c_int, c_ptr, c_int32_t
        type(c_ptr), value :: job

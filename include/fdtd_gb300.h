@@ -400,9 +400,14 @@ int fdtd_load_state(fdtd_job *job, const void *buf, uint64_t bytes);
  * fdtd_debug_fail_alloc makes the device allocation that follows `after`
  * further successful ones fail as an out-of-memory would, for any job of the
  * process (-1 switches it off): it lets a caller exercise its recovery from
- * FDTD_ENOMEM at every allocation of set-up and stepping. */
+ * FDTD_ENOMEM at every allocation of set-up and stepping.
+ * fdtd_debug_fail_launch does the same for the launches of the block-step
+ * kernels and the fused 3D step kernel: the one after `after` further ones is
+ * not made and reported as FDTD_ECUDA by the step (also where it captures a
+ * graph); a block-step kernel that fails while commit times it is left out. */
 int fdtd_check_finite(fdtd_job *job, int64_t *count);
 int fdtd_debug_fail_alloc(int32_t after);
+int fdtd_debug_fail_launch(int32_t after);
 /* fdtd_debug_wait_limit sets how many polls the TMA-staged 3D kernels (the
  * core kernels of tiles 7 and 8, and the fused step kernel of tile 9) make of
  * a copy's mbarrier before they give up on it (rounds < 0: the

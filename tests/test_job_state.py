@@ -76,3 +76,56 @@ def test_refused_load_state_leaves_the_state(gpu):
     assert np.any(J.get_field(abi.EZ))
     J.close()
     K.close()
+
+
+@pytest.mark.parametrize("dim", [1, 2, 3])
+def test_failed_launch_is_an_error_and_no_step(gpu, monkeypatch, dim):
+    """The first launch of a step fails: the step reports it, and the same call
+    again takes the step from the state before it."""
+    monkeypatch.setenv("FDTD_TUNE", "block")
+    if dim == 1:
+        spec, _ = problems.config_1d_gold(precision=abi.F32)
+        comps = (abi.EX, abi.HZ)
+    elif dim == 2:
+        spec, _ = problems.config_2d_tmz(precision=abi.F32, n=192, ncyl=2, nfreq=8, npml=16)
+        comps = FIELDS_TM
+    else:
+        spec, _ = problems.config_3d_sphere(precision=abi.F32, n=48, nfreq=4, npml=8)
+        comps = range(6)
+    outs = []
+    for fail in (False, True):
+        J = gpu.Job(spec)
+        J.step(1, 6)
+        if fail:
+            try:
+                gpu.fail_launch_after(0)
+                with pytest.raises(gpu.FdtdError) as e:
+                    J.step(7, 8)
+                assert e.value.code == abi.FDTD_ECUDA
+            finally:
+                gpu.fail_launch_after(-1)
+        J.step(7, 8)
+        J.step(15, 300)
+        outs.append(state_of(J, comps))
+        J.close()
+    assert any(np.any(a) for a in outs[0])
+    for a, b in zip(*outs):
+        np.testing.assert_array_equal(a, b)
+
+
+def test_kernel_that_fails_in_the_tuner_is_left_out(gpu):
+    spec, _ = problems.config_2d_tmz(precision=abi.F32, n=160, ncyl=1, nfreq=6, npml=12)
+    spec.materials = spec.materials[:1]  # a kind of grid of its own, not timed yet in this process
+    try:
+        gpu.fail_launch_after(0)
+        J = gpu.Job(spec)
+    finally:
+        gpu.fail_launch_after(-1)
+    assert J.tile() in (1, 2, 3)
+    J.step(1, 200)
+    K = gpu.Job(spec, tile=4)
+    K.step(1, 200)
+    for a, b in zip(state_of(J, FIELDS_TM), state_of(K, FIELDS_TM)):
+        np.testing.assert_array_equal(a, b)
+    J.close()
+    K.close()
