@@ -2602,6 +2602,7 @@ int ring_graph(fdtd_job *J) {
   if (!J->d_gate && (rc = alloc_dev(J, (void **)&J->d_gate, sizeof(int)))) return rc;
   CK(cudaStreamSynchronize(J->stream));
   const long long launches0 = J->launches;
+  const int pp0 = J->pp;  // recorded launches move nothing, whatever their number
   J->prog_prev = -1;  // events recorded outside the capture cannot be waited on inside it
   CK(cudaStreamBeginCapture(J->stream, cudaStreamCaptureModeThreadLocal));
   int bad = FDTD_OK;
@@ -2651,9 +2652,14 @@ int ring_graph(fdtd_job *J) {
   cudaGraph_t g = nullptr;
   cudaError_t e = cudaStreamEndCapture(J->stream, &g);
   J->prog_prev = -1;
+  J->pp = pp0;
   J->graph_kernels = (int)(J->launches - launches0);
   J->launches = launches0;
-  if (bad) { if (g) cudaGraphDestroy(g); return bad; }
+  if (bad) {
+    if (g) cudaGraphDestroy(g);
+    cudaGetLastError();  // of a capture that was cut short; the failure is reported here
+    return bad;
+  }
   if (e != cudaSuccess) return set_err(FDTD_ECUDA, "graph capture: %s", cudaGetErrorString(e));
   J->graph = g;
   e = cudaGraphInstantiate(&J->graph_exec, J->graph, 0);
@@ -3117,6 +3123,7 @@ int pack_capture(fdtd::Pack *P) {
   const cudaError_t e = cudaStreamEndCapture(P->stream, &g);
   if (bad != cudaSuccess || e != cudaSuccess) {
     if (g) cudaGraphDestroy(g);
+    cudaGetLastError();
     return set_err(FDTD_ECUDA, "pack graph capture: %s", cudaGetErrorString(bad != cudaSuccess ? bad : e));
   }
   P->graph = g;
@@ -3141,6 +3148,7 @@ int pack_capture_blocks(fdtd::Pack *P) {
     // the job's own stream and events carry its branch during the capture
     int *const own_base = J->d_base, *const own_half = J->d_half;
     const long long launches0 = J->launches;
+    const int pp0 = J->pp;
     bad = cudaStreamWaitEvent(J->stream, P->ev_fork, 0);
     J->d_base = P->d_n0 + q;
     J->d_half = nullptr;
@@ -3160,6 +3168,7 @@ int pack_capture_blocks(fdtd::Pack *P) {
     if (bad == cudaSuccess) bad = cudaStreamWaitEvent(P->stream, J->ev_fjoin, 0);
     kernels += (int)(J->launches - launches0);
     J->launches = launches0;
+    J->pp = pp0;
     J->d_base = own_base;
     J->d_half = own_half;
     J->prog_prev = -1;
@@ -3173,6 +3182,7 @@ int pack_capture_blocks(fdtd::Pack *P) {
   const cudaError_t e = cudaStreamEndCapture(P->stream, &g);
   if (rc || bad != cudaSuccess || e != cudaSuccess) {
     if (g) cudaGraphDestroy(g);
+    cudaGetLastError();
     return rc ? rc : set_err(FDTD_ECUDA, "pack graph capture: %s", cudaGetErrorString(bad != cudaSuccess ? bad : e));
   }
   P->graph = g;

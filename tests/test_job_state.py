@@ -129,3 +129,64 @@ def test_kernel_that_fails_in_the_tuner_is_left_out(gpu):
         np.testing.assert_array_equal(a, b)
     J.close()
     K.close()
+
+
+@pytest.mark.parametrize("dim,tile", [(2, 0), (3, 0), (3, 9)])
+@pytest.mark.parametrize("after", [1, 2])
+def test_failed_capture_leaves_the_state(gpu, monkeypatch, dim, tile, after):
+    """The capture of a ring of steps stops after an odd or even number of
+    recorded launches: nothing has run, so the job's fields are where they were."""
+    monkeypatch.setenv("FDTD_TUNE", "block")
+    if dim == 2:
+        spec, _ = problems.config_2d_tmz(precision=abi.F32, n=192, ncyl=2, nfreq=8, npml=16)
+        comps = FIELDS_TM
+    else:
+        spec, _ = problems.config_3d_sphere(precision=abi.F32, n=64, nfreq=4, npml=8)
+        comps = range(6)
+    outs = []
+    for fail in (False, True):
+        J = gpu.Job(spec, tile=tile)
+        if fail:
+            try:
+                gpu.fail_launch_after(after)
+                with pytest.raises(gpu.FdtdError) as e:
+                    J.step(1, 320)
+                assert e.value.code == abi.FDTD_ECUDA
+            finally:
+                gpu.fail_launch_after(-1)
+            assert all(not np.any(J.get_field(c)) for c in comps)
+        J.step(1, 320)
+        outs.append(state_of(J, comps))
+        J.close()
+    assert any(np.any(a) for a in outs[0])
+    for a, b in zip(*outs):
+        np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("after", [1, 5])
+def test_failed_pack_capture_leaves_the_members(gpu, monkeypatch, after):
+    """The capture of a pack's ring stops part way in its first or second job: the
+    members go on alone, from their own fields."""
+    from fdtd_gpu import serve
+    monkeypatch.setenv("FDTD_TUNE", "block")
+    specs = [problems.config_2d_tmz(precision=abi.F32, n=n, ncyl=2, nfreq=8, npml=16, seed=n)[0] for n in (160, 192)]
+    alone = []
+    for s in specs:
+        J = gpu.Job(s)
+        J.step(1, 900)
+        alone.append(state_of(J, FIELDS_TM))
+        J.close()
+    S = serve.Server(max_active=4, chunk_steps=64)
+    try:
+        gpu.fail_launch_after(after)
+        tickets = [S.submit(s, 900) for s in specs]
+        for tk, want in zip(tickets, alone):
+            assert S.wait(tk) == abi.REQ_DONE
+            got = state_of(S.job(tk), FIELDS_TM)
+            assert any(np.any(a) for a in want)
+            for a, b in zip(got, want):
+                np.testing.assert_array_equal(a, b)
+            S.release(tk)
+    finally:
+        gpu.fail_launch_after(-1)
+        S.close()
