@@ -281,7 +281,8 @@ struct fdtd_job {
   int vec = 1, cv0 = 0, cw = 0, cy0 = 0, ncore = 0, nedge = 0;
   int ch = 0, cz0 = 0, cd = 0;  // 3D: core box rows and planes
   int tile_req = 0, tile = 1;    // core block shape: requested (0: tune) and used
-  int split_tile = 1;            // of the split kernels beside the 3D block-step kernel
+  int split_tile = 1;            // of the split kernels beside a block-step kernel
+  int block_min = 1;             // least steps of a 2D block-step launch from the canonical field set
   int *d_edge = nullptr;
   cudaStream_t side[2] = {};
   cudaEvent_t ev_fork = nullptr, ev_join[2] = {};
@@ -1829,7 +1830,7 @@ void fill_common(fdtd_job *J, StepParams<T> &p) {
     p.cy0 = J->cy0;
     p.ch = J->ch;
     p.ncore = J->ncore;
-    p.tile = J->tile;
+    p.tile = J->tile == fused_tile(J) ? J->split_tile : J->tile;
     p.nedge = J->nedge;
     p.edge_units = J->d_edge;
   } else {
@@ -2244,7 +2245,8 @@ int tune_tiles(fdtd_job *J) {
     auto it = g_tune.find(key);
     if (it != g_tune.end()) {
       J->tile = it->second & 255;
-      J->split_tile = it->second >> 8;
+      J->split_tile = it->second >> 8 & 255;
+      J->block_min = it->second >> 16;
       return FDTD_OK;
     }
   }
@@ -2339,10 +2341,19 @@ int tune_tiles(fdtd_job *J) {
       cudaGetLastError();
       continue;
     }
-    if (J->dim == 3 && c < fused_tile(J) && ms < best_split) {
+    if (c < fused_tile(J) && ms < best_split) {
       best_split = ms;
       J->split_tile = c;
     }
+    // A 2D launch of k steps takes about (1/2 + k/16) of one of eight.  Fewer steps
+    // than pay for that run split, which is what a host that steps one by one gets
+    // (us a step, split / block with 1, 2, 3, 4 steps; TM with cylinders 512^2:
+    // 17 / 13 7 5 4, 1024^2: 15 / 21 12 10 8, 2048^2: 22 / 55 31 23 18, without them
+    // 21 / 34 19 15 12; 4096^2: 114 / 189 111 81 65; TE 8192^2: 520 / 1740 954 695 560).
+    // A split step called on its own takes 3 us more than the five timed in a row.
+    if (block && J->dim == 2)
+      for (J->block_min = 1; J->block_min < pl.ks && ms * pl.ks * (0.5f + J->block_min / 16.f) > J->block_min * (best + 0.015f);)
+        ++J->block_min;
     if (ms < best) {
       best = ms;
       choice = c;
@@ -2354,7 +2365,7 @@ int tune_tiles(fdtd_job *J) {
   J->tile = choice;
   if (failed) return FDTD_OK;  // the next job of the kind tries again
   std::lock_guard<std::mutex> lk(g_tune_mu);
-  g_tune[key] = choice | J->split_tile << 8;
+  g_tune[key] = choice | J->split_tile << 8 | J->block_min << 16;
   return FDTD_OK;
 }
 
@@ -2561,13 +2572,13 @@ template <typename T>
 int eager_steps(fdtd_job *J, int n, int left, int *done) {
   int rc;
   *done = 1;
-  // as many steps as a launch takes and the sample ring has room for; a single
-  // step of the 3D block-step kernel only to come back to the canonical field
-  // set (512^3: 2.1 ms against 1.7 split; the 256 x 256 x 384 column 0.36 and 0.30)
+  // as many steps as a launch takes and the sample ring has room for; too few of
+  // them only to come back to the canonical field set (a single 3D step, 512^3:
+  // 2.1 ms against 1.7 split; the 256 x 256 x 384 column 0.36 and 0.30)
   const int most = J->dim == 2 ? J->blk.ks : 2;
   const int k = std::min(std::min(left, most), kStageSteps - J->stage_fill);
   const bool block = fused_mode(J) && (J->dim == 2 || block3_mode(J));
-  if (block && (J->dim == 2 || k > 1 || J->pp)) {
+  if (block && (k >= (J->dim == 2 ? J->block_min : 2) || J->pp)) {
     if ((rc = J->dim == 2 ? block_step(J, n, k, J->stage_fill, false) : block3_step(J, n, k, J->stage_fill, false))) return rc;
     for (int s = 0; s < k; ++s)
       if ((rc = after_sample<T>(J, n + s))) return rc;

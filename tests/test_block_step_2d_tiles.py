@@ -32,3 +32,24 @@ def test_block_step_equals_half_steps(gpu, monkeypatch, te, nx, ny, kw):  # noqa
     assert split == 2 and any(np.any(r) for r in ref)
     for a, b in zip(got, ref):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("te", [False, True])
+def test_single_steps_of_a_large_grid_run_split(gpu, te):  # noqa: F811
+    """One step from the canonical field set takes the half-step kernels where the
+    block-step kernel's halo costs more (2048^2: 22 us against 55), and few
+    steps after an odd number of launches still come from the current set."""
+    spec = make(2048, 2048, te)
+    J = gpu.Job(spec)
+    if J.tile() == BLOCK:
+        J.profile()
+        for n in range(1, 9):
+            J.step(n, 1)
+        J.sync()
+        assert J.kernel_time(abi.KERNEL_E)[0] == 8 and J.kernel_time(abi.KERNEL_STEP)[0] == 0
+    J.close()
+    calls = (1, 1, 8, 1, 1, 2, 8, 3, 64, 1)
+    got, ref = result(gpu, spec, calls)[1], result(gpu, spec, (sum(calls),), tile=2)[1]
+    assert any(np.any(r) for r in ref)
+    for a, b in zip(got, ref):
+        np.testing.assert_array_equal(a, b)
