@@ -2989,9 +2989,9 @@ template <typename T>
 static int get_field_impl(fdtd_job *J, int comp, double *host) {
   if (comp < 0 || comp > 7 || !J->F[comp]) return set_err(FDTD_EINVAL, "component %d not in this layout", comp);
   const long long cnt = field_elems(J, comp);
-  if (const int rc = fused_settle(J)) return rc;
+  const void *from = J->pp && comp < 6 ? J->Fb[comp] : J->F[comp];  // the current set
   std::vector<T> tmp((size_t)cnt);
-  CK(cudaMemcpyAsync(tmp.data(), J->F[comp], (size_t)cnt * sizeof(T), cudaMemcpyDeviceToHost, J->stream));
+  CK(cudaMemcpyAsync(tmp.data(), from, (size_t)cnt * sizeof(T), cudaMemcpyDeviceToHost, J->stream));
   CK(cudaStreamSynchronize(J->stream));
   for (long long c = 0; c < cnt; ++c) host[c] = (double)tmp[(size_t)c];
   J->d2h += (uint64_t)cnt * sizeof(T);
