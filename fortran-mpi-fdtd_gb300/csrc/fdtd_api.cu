@@ -243,7 +243,7 @@ struct fdtd_job {
     int shape = 0, ks = 0, max_ade = 0, ntiles = 0, ngen = 0, scr_stride = 0;
     BlockGeom g{};
     Tile2 *tiles = nullptr;
-    uint16_t *sflags[2] = {};  // of plain and general tiles
+    uint32_t *sflags[2] = {};  // of plain and general tiles
     uint2 *ade = nullptr;
     void *scratch = nullptr;
     size_t bytes[5] = {};  // of the five buffers
@@ -1466,6 +1466,10 @@ void block_choose(const fdtd_job *J, BlockPlan &pl) {
 }
 
 void block_plan(const fdtd_job *J, BlockPlan &pl);
+template <typename T>
+void fill_common(fdtd_job *J, StepParams<T> &p);
+template <typename T>
+void set_sources(fdtd_job *J, StepParams<T> &p);
 
 // The plan of the 2D block-step kernel: tiles, the flags of their strips and
 // their dispersive cells; and the second set of buffers.
@@ -1507,14 +1511,17 @@ int setup_block(fdtd_job *J) {
     J->h2d += src ? bytes : 0;
     return FDTD_OK;
   };
+  StepParams<float> p;
+  fill_common<float>(J, p);
+  set_sources<float>(J, p);
   // every tile as a plain one: what its strips hold makes it plain or general
   if ((rc = upload(all.data(), (void **)&B.tiles, all.size() * sizeof(Tile2), 0))) return rc;
-  if ((rc = upload(nullptr, (void **)&B.sflags[0], (size_t)nt * sh.NA * sizeof(uint16_t), 1))) return rc;
-  launch_tile_flags(J->d_mat, J->d_rowflag, B.tiles, nt, sh.RA, sh.NA, sh.V, g, B.sflags[0], J->stream);
+  if ((rc = upload(nullptr, (void **)&B.sflags[0], (size_t)nt * sh.NA * sizeof(uint32_t), 1))) return rc;
+  launch_tile_flags(p, B.tiles, nt, sh.RA, sh.NA, sh.V, g, B.sflags[0], J->stream);
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(J->stream));
-  std::vector<uint16_t> sf((size_t)nt * sh.NA);
-  CK(cudaMemcpy(sf.data(), B.sflags[0], sf.size() * sizeof(uint16_t), cudaMemcpyDeviceToHost));
+  std::vector<uint32_t> sf((size_t)nt * sh.NA);
+  CK(cudaMemcpy(sf.data(), B.sflags[0], sf.size() * sizeof(uint32_t), cudaMemcpyDeviceToHost));
   std::vector<char> general((size_t)nt);
   for (int t = 0; t < nt; ++t) {
     unsigned f = 0;
@@ -1574,9 +1581,9 @@ int setup_block(fdtd_job *J) {
       std::sort(ade.begin() + t.ade0, ade.begin() + t.ade0 + t.nade,
                 [](const uint2 &x, const uint2 &y) { return (x.y & 0xffffu) < (y.y & 0xffffu); });
   if ((rc = upload(tiles.data(), (void **)&B.tiles, tiles.size() * sizeof(Tile2), 0))) return rc;
-  if ((rc = upload(nullptr, (void **)&B.sflags[1], (size_t)std::max(1, ngen) * sh.NB * sizeof(uint16_t), 2))) return rc;
-  launch_tile_flags(J->d_mat, J->d_rowflag, B.tiles + ngen, nt - ngen, sh.RA, sh.NA, sh.V, g, B.sflags[0], J->stream);
-  launch_tile_flags(J->d_mat, J->d_rowflag, B.tiles, ngen, sh.RB, sh.NB, sh.V, g, B.sflags[1], J->stream);
+  if ((rc = upload(nullptr, (void **)&B.sflags[1], (size_t)std::max(1, ngen) * sh.NB * sizeof(uint32_t), 2))) return rc;
+  launch_tile_flags(p, B.tiles + ngen, nt - ngen, sh.RA, sh.NA, sh.V, g, B.sflags[0], J->stream);
+  launch_tile_flags(p, B.tiles, ngen, sh.RB, sh.NB, sh.V, g, B.sflags[1], J->stream);
   CK(cudaGetLastError());
   if ((rc = upload(ade.data(), (void **)&B.ade, ade.size() * sizeof(uint2), 3))) return rc;
   if (s0 > 0 &&
@@ -1644,9 +1651,6 @@ int setup_fused3(fdtd_job *J) {
   J->fused_ok = true;
   return FDTD_OK;
 }
-
-template <typename T>
-void fill_common(fdtd_job *J, StepParams<T> &p);
 
 // The 3D block-step kernel takes any FP32 grid of even row length without
 // reference slabs or a TFSF box (those update fields in place), and materials
@@ -3926,9 +3930,9 @@ int fdtd_estimate_bytes(const fdtd_job *J, uint64_t *bytes) {
     b += J->probes.size() * 360ull * w;
   }
   // the 2D block-step kernel's: the fields and the stored PML part, its tiles
-  // (at least 112 x 16 cells, 96 bytes with their flags)
+  // (at least 112 x 16 cells, 160 bytes with their flags)
   const bool block2 = J->dim == 2 && w == 4 && !J->has_tfbox && !J->lean && !(J->has_pml && J->pml.mode == FDTD_PML_REFERENCE);
-  if (block2) b += 4 * N * w + ((uint64_t)nx / 112 + 1) * ((uint64_t)ny / 16 + 1) * 96;
+  if (block2) b += 4 * N * w + ((uint64_t)nx / 112 + 1) * ((uint64_t)ny / 16 + 1) * 160;
   if (J->dim == 1 && !J->lean)  // the 1D block-step kernel's second set and slot map
     b += (J->has_tfsf ? 4 : 2) * N * w + 4 * N + 8ull * (J->pml.npml[1][0] + 2) * w;
   if (J->has_tfsf) b += 2 * N * w;

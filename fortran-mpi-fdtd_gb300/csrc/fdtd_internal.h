@@ -277,8 +277,8 @@ struct Tile2 {
   int pad;
 };
 // flags of a tile's warp strips: cells that are not main cells, main cells of
-// several materials or dispersive ones, rows with a source, rows with a sample,
-// split-PML cells
+// several materials or dispersive ones, cells with a source, owned columns with a
+// sample, split-PML cells
 enum StripFlag : int { SF_GEN = 1, SF_MIX = 2, SF_SRC = 4, SF_SMP = 8, SF_SHELL = 16 };
 // tiles of ox cells by oy rows, widened by hx cells and hy rows
 struct BlockGeom {
@@ -292,7 +292,7 @@ struct BlockGeom {
 struct BlockPlan {
   const Tile2 *tiles;     // the general ones (any cells, sources, samples) first
   int ngen;
-  const uint16_t *sflags[2];  // plain, general: per tile and warp StripFlag bits, material id << 8
+  const uint32_t *sflags[2];  // plain, general: per tile and warp StripFlag bits, material id << 8, sampled rows << 16
   const uint2 *ade;       // x: slot, bit 31: the tile owns the cell; y: cell in the tile, material id << 16
   BlockGeom g;
   int ntiles;
@@ -320,8 +320,8 @@ BlockShape block_shape(int shape);
 void block_smem(BlockPlan &pl, int layout, int max_ade, bool split, bool smp_rows);
 // the general or the plain tiles of a launch; returns the kernels launched, -1 on failure
 int launch_step2d_block(const StepParams<float> &p, const BlockPlan &pl, bool gen, void *stream);
-void launch_tile_flags(const uint8_t *mat, const uint8_t *rowflag, const Tile2 *tiles, int ntiles, int R, int NW, int V,
-                       const BlockGeom &g, uint16_t *out, void *stream);
+void launch_tile_flags(const StepParams<float> &p, const Tile2 *tiles, int ntiles, int R, int NW, int V, const BlockGeom &g,
+                       uint32_t *out, void *stream);
 
 // packs of 2D jobs: one launch runs one part of every job's half step
 constexpr int kMaxPack = 32;

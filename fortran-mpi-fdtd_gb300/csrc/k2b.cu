@@ -50,10 +50,25 @@ __device__ __forceinline__ int wrap_i(int i, int n) {
   return i < 0 ? i + n : i;
 }
 
+// whether the cells lo..hi of row j hold a sample (mons: monitors count)
+__device__ __forceinline__ bool row_sampled(const StepParams<T> &p, int j, int lo, int hi, bool mons = true) {
+  for (int q = 0; mons && q < p.nmon; ++q) {
+    const Monitor &m = p.mon[q];
+    if (j >= m.lo[1] && j <= m.hi[1] && hi >= m.lo[0] && lo <= m.hi[0]) return true;
+  }
+  for (int q = 0; q < p.nprobe; ++q)
+    if (p.probe[q].cell[1] == j && p.probe[q].cell[0] >= lo && p.probe[q].cell[0] <= hi) return true;
+  return false;
+}
+
 // Flags (SF_*) of the warp strips of the plan's tiles, from the material ids and
 // the set-up's ranges, with the id of a strip's main cells where they have one.
-__global__ void tile_flags_kernel(const uint8_t *mat, const uint8_t *rowflag, const Tile2 *tiles, int ntiles, int R, int NW,
-                                  int W, BlockGeom g, uint16_t *out) {
+// Sources count where one of the strip's cells is driven, samples where an owned
+// cell is: by rows alone a vertical line of either would make every tile of the
+// grid a general one (2048^2 with a square of line monitors: 43.9 us a step, 13.9
+// like this; the half-step kernels 27.7).
+__global__ void tile_flags_kernel(const __grid_constant__ StepParams<T> p, const Tile2 *tiles, int ntiles, int R, int NW,
+                                  int W, BlockGeom g, uint32_t *out) {
   const int strip = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (strip >= ntiles * NW) return;
   const int t = strip / NW, w = strip % NW;
@@ -64,8 +79,8 @@ __global__ void tile_flags_kernel(const uint8_t *mat, const uint8_t *rowflag, co
     int j = y0 + r;
     if (g.per[1]) j = wrap_i(j, g.ny);
     const bool jin = j >= 0 && j < g.ny;
-    if (jin && (rowflag[j] & ROW_SRC)) f |= SF_SRC;
-    if (jin && (rowflag[j] & ROW_SAMPLE)) f |= SF_SMP;
+    const int rf = jin ? p.rowflag[j] : 0, xo = tiles[t].tx * g.ox;
+    if ((rf & ROW_SAMPLE) && row_sampled(p, j, xo, min(xo + g.ox, g.nx) - 1)) f |= SF_SMP | 0x10000u << r;
     for (int x = lane; x < W; x += 32) {
       int i = x0 + x;
       if (g.per[0]) i = wrap_i(i, g.nx);
@@ -74,8 +89,11 @@ __global__ void tile_flags_kernel(const uint8_t *mat, const uint8_t *rowflag, co
       const bool main = in && !shell && i >= g.mlo[0] && i <= g.mhi[0] && j >= g.mlo[1] && j <= g.mhi[1];
       if (!main) f |= SF_GEN;
       if (shell) f |= SF_SHELL;
+      if (in && (rf & ROW_SRC))
+        for (int q = 0; q < p.nsrc; ++q)
+          if (i >= p.src[q].lo[0] && i <= p.src[q].hi[0] && j >= p.src[q].lo[1] && j <= p.src[q].hi[1]) f |= SF_SRC;
       if (main) {
-        const int id = mat[(long long)j * g.nx + i];
+        const int id = p.mat[(long long)j * g.nx + i];
         lo = min(lo, id);
         hi = max(hi, id);
       }
@@ -87,7 +105,7 @@ __global__ void tile_flags_kernel(const uint8_t *mat, const uint8_t *rowflag, co
     hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
   }
   if (hi >= 0 && (lo != hi || hi >= kAdeId)) f |= SF_MIX;
-  if (lane == 0) out[strip] = (uint16_t)(f | (unsigned)(hi < 0 || (f & SF_MIX) ? g.id0 : hi) << 8);
+  if (lane == 0) out[strip] = f | (unsigned)(hi < 0 || (f & SF_MIX) ? g.id0 : hi) << 8;
 }
 
 // One tile.  GEN: any cells, sources and samples; else every cell is a main cell
@@ -104,7 +122,7 @@ __device__ __forceinline__ void block_tile(const StepParams<T> &p, const BlockPl
   constexpr int W = 32 * V, H = R * NW, NT = 32 * NW;
   constexpr int NC = L == 3 ? 1 : 2;            // E components
   constexpr bool TM = L == 3;
-  static_assert(R * V <= 32, "a thread's cells are bits of one word");
+  static_assert(R * V <= 32 && (!GEN || R * (V + 1) <= 32), "a thread's cells are bits of one word");
   extern __shared__ __align__(16) unsigned char sm_raw[];
   T *const topH = (T *)sm_raw, *const botE = topH + NW * W;
   T *const xsm = botE + NW * W, *const ysm = xsm + 4 * W;  // PML profiles f1 f2 g1 g2 along the tile's x and y
@@ -123,8 +141,8 @@ __device__ __forceinline__ void block_tile(const StepParams<T> &p, const BlockPl
   // samples of the launch's steps, [step][row][field][W]: at most kBlockRows rows
   T *const smp = (T *)(sm_raw + pl.off_smp);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const uint16_t *const sflags = pl.sflags[GEN] + blockIdx.x * NW;
-  const unsigned sf = sflags[w];  // flags, and the id of the strip's main cells << 8
+  const uint32_t *const sflags = pl.sflags[GEN] + blockIdx.x * NW;
+  const unsigned sf = sflags[w];  // flags, the id of the strip's main cells << 8, rows with samples << 16
   const int nx = p.nx, ny = p.ny;
   const int xr = tl.tx * pl.g.ox - pl.g.hx + lane * V;  // the thread's first cell and first row, unwrapped
   const int yr = tl.y0 - pl.g.hy + w * R;
@@ -162,7 +180,7 @@ __device__ __forceinline__ void block_tile(const StepParams<T> &p, const BlockPl
     const int ly = w * R + r;
     return ly >= pl.g.hy && ly < pl.g.hy + tl.oy && yr + r < ny;
   };
-  const T cas = __ldg(p.mca + (sf >> 8));  // Ku/eps of a strip of one material
+  const T cas = __ldg(p.mca + (sf >> 8 & 0xffu));  // Ku/eps of a strip of one material
   // this strip or the one above it may hold dispersive cells
   const bool near = GEN && tl.nade > 0 && ((sf | (w + 1 < NW ? sflags[w + 1] : 0u)) & SF_MIX);
   // rows with a source, and owned rows with samples
@@ -171,15 +189,14 @@ __device__ __forceinline__ void block_tile(const StepParams<T> &p, const BlockPl
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       const int j = row_j(r);
-      const int rf = j >= 0 && j < ny ? __ldg(p.rowflag + j) : 0;
-      if (rf & ROW_SRC) srow |= 1u << r;
-      if ((rf & ROW_SAMPLE) && p.gather && row_own(r)) grow |= 1u << r;
+      if ((sf & SF_SRC) && j >= 0 && j < ny && (__ldg(p.rowflag + j) & ROW_SRC)) srow |= 1u << r;
+      if ((sf >> (16 + r) & 1u) && p.gather && row_own(r)) grow |= 1u << r;
     }
   // a strip of one material driven by the job's one source
   unsigned srcm = 0;
   T css = T(0);
   if (GEN && p.nsrc == 1 && srow && !(sf & SF_MIX)) {
-    css = __ldg(p.mcs + (sf >> 8));
+    css = __ldg(p.mcs + (sf >> 8 & 0xffu));
     const Source &sr = p.src[0];
 #pragma unroll
     for (int r = 0; r < R; ++r)
@@ -331,6 +348,17 @@ __device__ __forceinline__ void block_tile(const StepParams<T> &p, const BlockPl
     if (nsrow <= kBlockRows && lane == 0)
       for (unsigned m = grow, k = srow0; m; m &= m - 1, ++k) rowj[k] = yr + __ffs(m) - 1;
   }
+  // the thread's cells that are taken one by one: a line along y is one cell of
+  // four in a row, and the loop over them is what a tile with such a line waits for
+  // (bits of grow above its rows': the loop has no register to spare)
+  if (GEN && grow && (nsrow > kBlockRows || p.nprobe > 0))
+#pragma unroll 1
+    for (unsigned m = grow; m; m &= m - 1) {
+      const int rr = __ffs(m) - 1;
+#pragma unroll 1
+      for (int q = 0; q < V; ++q)
+        if (((xow >> q) & 1u) && row_sampled(p, yr + rr, xr + q, xr + q, nsrow > kBlockRows)) grow |= 1u << (R + rr * V + q);
+    }
   if (GEN && KIND != MK_GOLD && adem) {  // their E before the first step
 #pragma unroll
     for (int r = 0; r < R; ++r)
@@ -639,24 +667,21 @@ __device__ __forceinline__ void block_tile(const StepParams<T> &p, const BlockPl
           }
       }
 #pragma unroll 1
-      for (unsigned m = nsrow > kBlockRows || p.nprobe > 0 ? grow : 0u; m; m &= m - 1) {
-        const int rr = __ffs(m) - 1, j = yr + rr;
-#pragma unroll 1
-        for (int q = 0; q < V; ++q) {
-          if (!((xow >> q) & 1u)) continue;
-          T va = T(0), vb = T(0), vc = T(0);
+      for (unsigned m = __reduce_or_sync(0xffffffffu, grow >> R); m; m &= m - 1) {
+        const int at = __ffs(m) - 1;
+        if (!((grow >> (R + at)) & 1u)) continue;
+        T va = T(0), vb = T(0), vc = T(0);
 #pragma unroll
-          for (int r = 0; r < R; ++r)
+        for (int r = 0; r < R; ++r)
 #pragma unroll
-            for (int u = 0; u < V; ++u)
-              if (r == rr && u == q) {
-                va = a[r][u];
-                vb = b[r][u];
-                vc = c[r][u];
-              }
-          const T vals[6] = {TM ? T(0) : va, TM ? T(0) : vb, TM ? va : T(0), TM ? vb : T(0), TM ? vc : T(0), TM ? T(0) : vc};
-          gather_cell<T>(p, n, xr + q, j, 0, vals, p.slot + s, nsrow > kBlockRows);
-        }
+          for (int u = 0; u < V; ++u)
+            if (r * V + u == at) {
+              va = a[r][u];
+              vb = b[r][u];
+              vc = c[r][u];
+            }
+        const T vals[6] = {TM ? T(0) : va, TM ? T(0) : vb, TM ? va : T(0), TM ? vb : T(0), TM ? vc : T(0), TM ? T(0) : vc};
+        gather_cell<T>(p, n, xr + at % V, yr + at / V, 0, vals, p.slot + s, nsrow > kBlockRows);
       }
     }
   }
@@ -808,11 +833,11 @@ int launch_step2d_block(const StepParams<T> &p, const BlockPlan &pl, bool gen, v
   return pl.shape == 0 ? launch_block_s<2, 0>(p, pl, gen, s) : launch_block_s<2, 1>(p, pl, gen, s);
 }
 
-void launch_tile_flags(const uint8_t *mat, const uint8_t *rowflag, const Tile2 *tiles, int ntiles, int R, int NW, int V,
-                       const BlockGeom &g, uint16_t *out, void *stream) {
+void launch_tile_flags(const StepParams<T> &p, const Tile2 *tiles, int ntiles, int R, int NW, int V, const BlockGeom &g,
+                       uint32_t *out, void *stream) {
   const int strips = ntiles * NW;
   if (strips <= 0) return;
-  tile_flags_kernel<<<(strips + 7) / 8, 256, 0, (cudaStream_t)stream>>>(mat, rowflag, tiles, ntiles, R, NW, 32 * V, g, out);
+  tile_flags_kernel<<<(strips + 7) / 8, 256, 0, (cudaStream_t)stream>>>(p, tiles, ntiles, R, NW, 32 * V, g, out);
 }
 
 }  // namespace fdtd

@@ -53,3 +53,29 @@ def test_single_steps_of_a_large_grid_run_split(gpu, te):  # noqa: F811
     assert any(np.any(r) for r in ref)
     for a, b in zip(got, ref):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("te", [False, True])
+@pytest.mark.parametrize("nx,ny,kw", [
+    (1345, 673, {}), (560, 300, {}), (449, 131, dict(pml=0, per=(1, 1), lorentz=True)), (225, 96, dict(per=(1, 0))),
+])
+def test_columns_of_samples_and_sources(gpu, monkeypatch, te, nx, ny, kw):  # noqa: F811
+    """Line monitors and sources along y and probes, on and beside the first and
+    last column that a tile owns (112 of them) and at the ends of the grid."""
+    monkeypatch.setenv("FDTD_TUNE", "block")
+    spec = make(nx, ny, te, **kw)
+    e, h = (abi.EX, abi.HZ) if te else (abi.EZ, abi.HX)
+    om = spec.monitors[0].omega
+    for x in (0, 111, 112, 223, nx - 1):
+        spec.add_monitor((x, 3, 0), (x, ny - 4, 0), (e, h), om)
+        spec.add_probe((x, ny // 2, 0), (e, h))
+    spec.add_monitor((100, 20, 0), (130, 40, 0), (h, e), om)
+    for x in (lo for lo in (spec.main_lo[0], 105, 112) if lo <= spec.main_hi[0]):
+        spec.sources.append(dict(component=e, lo=(x, 5, 0), hi=(x, ny - 6, 0), amp=0.3, t0=1e-16, st=2e-16, w0=3e15))
+    calls = (3, 8, 64, 17, 31)
+    used, got = result(gpu, spec, calls)
+    assert used == BLOCK
+    ref = result(gpu, spec, (sum(calls),), tile=2)[1]
+    for a, b in zip(got, ref):
+        assert np.any(b)
+        np.testing.assert_array_equal(a, b)
