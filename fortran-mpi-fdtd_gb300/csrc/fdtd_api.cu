@@ -20,6 +20,7 @@
 #include <nvtx3/nvToolsExt.h>
 
 #include <algorithm>
+#include <array>
 #include <atomic>
 #include <cmath>
 #include <complex>
@@ -251,6 +252,7 @@ struct fdtd_job {
   // the 3D block-step kernel: its tiles and tables, and the second sets of the
   // stored split-PML parts
   bool block3_ok = false;
+  int b3_mixed = 0;  // eighths of its rows with cells of more than the most common material
   bool lean = false;  // leave out every kernel that needs second sets of buffers
   Block3 b3{};
   void *spb3[6] = {};
@@ -1685,11 +1687,13 @@ int setup_block3(fdtd_job *J) {
   std::vector<int> order((size_t)nt);
   std::vector<long long> weight((size_t)nt, 0);
   std::vector<char> ade((size_t)nt, 0);
+  size_t mixed = 0;
   for (int k = 0; k < J->nz; ++k)
     for (int j = 0; j < J->ny; ++j)
       for (int tx = 0; tx < b.ntx; ++tx) {
         const uint8_t f = fl[((size_t)k * J->ny + j) * b.ntx + tx];
         weight[((size_t)(k / b.oz) * b.nty + j / b.oy) * b.ntx + tx] += f & 4 ? 4 : f & 0x11 ? 1 : 0;
+        mixed += f & 4 ? 1 : 0;
         if (f & 64)  // in every tile whose halo reaches the row
           tiles_of(k, J->nz, J->g.periodic[2], b.oz, 2, b.oz + 4, [&](int tz, int, bool) {
             tiles_of(j, J->ny, J->g.periodic[1], b.oy, 1, b.oy + 3, [&](int ty, int, bool) { ade[((size_t)tz * b.nty + ty) * b.ntx + tx] = 1; });
@@ -1697,6 +1701,7 @@ int setup_block3(fdtd_job *J) {
       }
   for (int t = 0; t < nt; ++t) order[t] = t;
   for (char c : ade) b.nade += c;
+  J->b3_mixed = (int)(8 * mixed / rows);
   std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
     return ade[x] != ade[y] ? ade[x] > ade[y] : weight[x] / 64 > weight[y] / 64;
   });
@@ -2141,7 +2146,7 @@ int run_parts(fdtd_job *J, const StepParams<T> &p, const bool (&want)[3], bool e
 // the fastest is kept.  The choice is cached per kind of grid (dimension,
 // layout, precision, vector width, log2 of the core cells).
 std::mutex g_tune_mu;
-std::map<long long, int> g_tune;
+std::map<std::array<long long, 2>, int> g_tune;
 
 // the block-step launch's two sets of buffers: step n in set `from`, the new
 // step to the other
@@ -2236,14 +2241,19 @@ int tune_tiles(fdtd_job *J) {
   }
   int lg = 0;
   for (long long c = J->ncore; c > 1; c >>= 1) ++lg;
-  // which TMA-staged kernels the grid can take, and the share of dispersive
-  // cells (halvings, up to 15), are part of the kind of grid
+  // which TMA-staged kernels the grid can take, the share of dispersive cells
+  // (halvings, up to 15), their update, and the share (in eighths) of 2D tiles or
+  // 3D rows that the block-step kernel cannot take as plain ones are part of the
+  // kind of grid: plain 320^3 runs 437 us a step in that kernel and 493 split, of
+  // two mixed materials 810 and 511
   int lade = 0;
   for (long long c = J->nade; lade < 15 && c < J->ncore; c *= 2, ++lade)
     if (c == 0) { lade = 15; break; }
-  const long long key = ((((((long long)J->dim * 8 + J->g.layout) * 4 + J->g.precision) * 8 + J->vec) * 64 + lg) * 16 + lade) * 8 +
-                        (J->fused_ok ? 4 : 0) + (J->tma_ok ? 2 : 0) + (J->tma_ok && J->tma.h_ok ? 1 : 0) +
-                        (J->block3_ok ? 1ll << 40 : 0);
+  const long long mixed = J->dim == 2 && J->fused_ok ? 8ll * J->blk.ngen / std::max(1, J->blk.ntiles) : J->b3_mixed;
+  const std::array<long long, 2> key = {
+      ((((((long long)J->dim * 8 + J->g.layout) * 4 + J->g.precision) * 8 + J->vec) * 64 + lg) * 16 + lade) * 8 +
+          (J->fused_ok ? 4 : 0) + (J->tma_ok ? 2 : 0) + (J->tma_ok && J->tma.h_ok ? 1 : 0),
+      ((J->ade_kind + 1ll) * 16 + mixed) * 4 + (J->ac_host.size() > sizeof(AdeCoef<T>) ? 2 : 0) + (J->block3_ok ? 1 : 0)};
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     auto it = g_tune.find(key);
