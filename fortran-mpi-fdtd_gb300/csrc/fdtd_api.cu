@@ -2249,11 +2249,20 @@ int tune_tiles(fdtd_job *J) {
   int lade = 0;
   for (long long c = J->nade; lade < 15 && c < J->ncore; c *= 2, ++lade)
     if (c == 0) { lade = 15; break; }
+  // and how well the grid fills the 3D block-step kernel's tiles (sixteenths of the
+  // cells of its rounds: 320 x 320 x 200 411 us a step there and 315 split, 320 x
+  // 240 x 300, of as many cells, 279 and 353)
+  long long fill = 0;
+  if (J->block3_ok) {
+    const Block3 &b = J->b3;
+    const long long waves = ((long long)b.ntx * b.nty * b.ntz + J->num_sms - 1) / J->num_sms;
+    fill = 16ll * J->ncell / (waves * (b.oz + 6) * J->num_sms * b.ox * b.oy);
+  }
   const long long mixed = J->dim == 2 && J->fused_ok ? 8ll * J->blk.ngen / std::max(1, J->blk.ntiles) : J->b3_mixed;
   const std::array<long long, 2> key = {
       ((((((long long)J->dim * 8 + J->g.layout) * 4 + J->g.precision) * 8 + J->vec) * 64 + lg) * 16 + lade) * 8 +
           (J->fused_ok ? 4 : 0) + (J->tma_ok ? 2 : 0) + (J->tma_ok && J->tma.h_ok ? 1 : 0),
-      ((J->ade_kind + 1ll) * 16 + mixed) * 4 + (J->ac_host.size() > sizeof(AdeCoef<T>) ? 2 : 0) + (J->block3_ok ? 1 : 0)};
+      (((J->ade_kind + 1ll) * 16 + mixed) * 32 + fill) * 4 + (J->ac_host.size() > sizeof(AdeCoef<T>) ? 2 : 0) + (J->block3_ok ? 1 : 0)};
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     auto it = g_tune.find(key);
@@ -2346,7 +2355,20 @@ int tune_tiles(fdtd_job *J) {
   for (int c = 0; c <= last; ++c) {
     if (c >= nshapes && c < kBlock3Tile) continue;
     const bool block = (J->dim == 2 && c == fused_tile(J)) || (J->dim == 3 && c == kBlock3Tile);
-    if (block) best = time5(split_step);
+    if (block) {
+      best = time5(split_step);
+      // 3D: the fused kernel may be the best core and yet lose with the edges that
+      // it leaves to others (256 x 256 x 128: 178 us a step, the split shape 143)
+      if (J->dim == 3 && choice == fused_tile(J)) {
+        const float fused = best;
+        choice = J->split_tile;
+        best = time5(split_step);
+        if (fused < best) {
+          best = fused;
+          choice = fused_tile(J);
+        }
+      }
+    }
     p.tile = c;
     float ms = time5([&] { cores(c); }) / (block ? (float)(J->dim == 2 ? pl.ks : 2) : 1.f);  // of a step
     // (the first runs of the 3D block-step kernel take a quarter longer than all later ones)
@@ -2368,7 +2390,9 @@ int tune_tiles(fdtd_job *J) {
     if (block && J->dim == 2)
       for (J->block_min = 1; J->block_min < pl.ks && ms * pl.ks * (0.5f + J->block_min / 16.f) > J->block_min * (best + 0.015f);)
         ++J->block_min;
-    if (ms < best) {
+    // (in a replayed graph a split step is a few per cent shorter than here: 200^3
+    // 142 us, where the 3D block-step kernel takes 145)
+    if (ms * (J->dim == 3 && block ? 1.05f : 1.0f) < best) {
       best = ms;
       choice = c;
     }
