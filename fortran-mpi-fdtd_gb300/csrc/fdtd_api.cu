@@ -36,6 +36,7 @@
 #include "fdtd_gb300.h"
 #include "fdtd_internal.h"
 #include "hostscan.h"
+#include "hosttiles.h"
 
 using namespace fdtd;
 
@@ -347,12 +348,10 @@ int alloc_dev(fdtd_job *J, void **p, size_t bytes) {
   if (e != cudaSuccess) return set_err(FDTD_ENOMEM, "device allocation of %zu bytes: %s", bytes, cudaGetErrorString(e));
   J->allocs.push_back(*p);
   J->dev_bytes += bytes;
+  // the buffer is ready in the order of the job's stream, which everything that
+  // touches it is on or waits for (a wait here each time: 0.1-0.3 ms of a commit)
   e = cudaMemsetAsync(*p, 0, bytes, J->stream);
   if (e != cudaSuccess) return set_err(FDTD_ECUDA, "cudaMemsetAsync: %s", cudaGetErrorString(e));
-  // the buffer is ready only in the job stream's order: wait for it (and its
-  // zeroing) before uploads on other streams or the host may touch it
-  e = cudaStreamSynchronize(J->stream);
-  if (e != cudaSuccess) return set_err(FDTD_ECUDA, "cudaStreamSynchronize: %s", cudaGetErrorString(e));
   return FDTD_OK;
 }
 
@@ -646,6 +645,14 @@ size_t ade_bytes(const fdtd_job *J);
 int fused_tile(const fdtd_job *J) { return J->dim == 3 ? 8 : 3; }
 constexpr int kBlock3Tile = 9;
 void free_block3(fdtd_job *J);
+// The 3D block-step kernel loses on small grids, whose tiles are few and mostly
+// halo and shell (us a step, block / split: 160^3 123 / 80, 200^3 160 / 143, 128 x
+// 128 x 384 99 / 93; 160 x 160 x 384, 9.8 million cells, 125 / 148), so jobs below
+// six million cells neither set it up nor count its buffers.
+bool block3_worth(const fdtd_job *J) {
+  const char *e = getenv("FDTD_TUNE");
+  return J->ncell >= 6000000 || (e && e[0] == 'b');
+}
 
 // The TFSF box: faces, and the cells its face terms touch (the box widened by
 // one cell across each face) inside the grid, the main range and the PML's
@@ -1433,25 +1440,6 @@ void free_block3(fdtd_job *J) {
 // bytes of the dispersive state
 size_t ade_bytes(const fdtd_job *J) { return J->esz * (size_t)std::max(1, J->ade_nf) * 3 * std::max(32, J->ade_stride); }
 
-// The tiles of width `len` (o cells owned, h of halo) that hold cell i of an
-// axis of n cells: calls f(tile, place in the tile, whether the tile owns it).
-// On a periodic axis the halo wraps, so a tile may hold images of a cell.
-template <typename F>
-void tiles_of(int i, int n, bool per, int o, int h, int len, F f) {
-  const int nt = (n + o - 1) / o;
-  const int lo = -h, hi = (nt - 1) * o - h + len;  // the span of all tiles
-  const int m0 = per ? -((i - lo) / n) : 0, m1 = per ? (hi - 1 - i) / n : 0;
-  for (int m = m0; m <= m1; ++m) {
-    const int x = i + m * n;
-    if (x < lo || x >= hi) continue;
-    const int t0 = std::max(0, (x + h - len + 1 + o - 1) / o), t1 = std::min(nt - 1, (x + h) / o);
-    for (int t = t0; t <= t1; ++t) {
-      const int l = x - (t * o - h);
-      if (l >= 0 && l < len) f(t, l, m == 0 && l >= h && l < h + o);
-    }
-  }
-}
-
 // The shape and the steps per launch of the 2D block-step kernel.  8 steps: half
 // the launches, loads and stores of 4 for 1.2 times the halo's arithmetic (2048^2
 // with 40 cylinders: 12.3 against 16.9 us a step; 256^2: 2.5 against 4.2).  64-row
@@ -1531,17 +1519,26 @@ int setup_block(fdtd_job *J) {
     general[t] = f != 0;
     all[t].smp = f & SF_SMP ? 1 : 0;
   }
-  // f(cell, tile, place in the tile, whether the tile owns it) of the dispersive cells
+  // f(first cell, cells, tile, place of the first in the tile, from which to which
+  // of them the tile owns) of the dispersive cells, a stretch of a row at a time;
+  // they are in the order of the grid
   auto each = [&](auto f) {
-    for (int q = 0; q < J->nade; ++q) {
-      const int i = J->ade_cell_host[q] % J->nx, j = J->ade_cell_host[q] / J->nx;
+    for (int q = 0, r; q < J->nade; q = r) {
+      const int c = J->ade_cell_host[q], j = c / J->nx, i = c - j * J->nx;
+      const int most = std::min(J->nade, q + J->nx - i);  // to the row's end
+      for (r = q + 1; r < most && J->ade_cell_host[r] == c + (r - q);) ++r;
       tiles_of(j, J->ny, g.per[1], g.oy, g.hy, H, [&](int ty, int ly, bool oy) {
-        tiles_of(i, J->nx, g.per[0], g.ox, g.hx, W, [&](int tx, int lx, bool ox) { f(q, ty * ntx + tx, ly * W + lx, ox && oy); });
+        stretches_of(i, r - q, J->nx, g.per[0], g.ox, g.hx, W, [&](int tx, int skip, int n, int lx, int own0, int own1) {
+          f(q + skip, n, ty * ntx + tx, ly * W + lx, oy ? own0 : 0, oy ? own1 : 0);
+        });
       });
     }
   };
   long long total = 0;
-  each([&](int, int t, int, bool) { ++all[t].nade; ++total; });
+  each([&](int, int n, int t, int, int, int) {
+    all[t].nade += n;
+    total += n;
+  });
   if (total > INT32_MAX) {
     free_fused(J);
     return FDTD_OK;  // not offered
@@ -1572,11 +1569,13 @@ int setup_block(fdtd_job *J) {
   }
   B.scr_stride = s0;
   std::vector<uint2> ade((size_t)std::max(1, a0));
-  each([&](int q, int t, int l, bool own) {
-    uint2 e;
-    e.x = (unsigned)q | (own ? 0x80000000u : 0u);
-    e.y = (unsigned)l | (unsigned)J->ade_mat_host[q] << 16;
-    ade[at[t]++] = e;
+  each([&](int q, int n, int t, int l, int own0, int own1) {
+    uint2 *const e = ade.data() + at[t];
+    at[t] += n;
+    for (int u = 0; u < n; ++u) {
+      e[u].x = (unsigned)(q + u) | (u >= own0 && u < own1 ? 0x80000000u : 0u);
+      e[u].y = (unsigned)(l + u) | (unsigned)J->ade_mat_host[q + u] << 16;
+    }
   });
   if (g.per[0] || g.per[1])  // the halo's images come out of order
     for (const Tile2 &t : tiles)
@@ -1688,17 +1687,26 @@ int setup_block3(fdtd_job *J) {
   std::vector<long long> weight((size_t)nt, 0);
   std::vector<char> ade((size_t)nt, 0);
   size_t mixed = 0;
+  size_t smp0 = rows, smp1 = 0;  // from the first to past the last row with samples
   for (int k = 0; k < J->nz; ++k)
-    for (int j = 0; j < J->ny; ++j)
+    for (int j = 0; j < J->ny; ++j) {
+      const size_t r0 = ((size_t)k * J->ny + j) * b.ntx;
+      long long *const w = weight.data() + ((size_t)(k / b.oz) * b.nty + j / b.oy) * b.ntx;
       for (int tx = 0; tx < b.ntx; ++tx) {
-        const uint8_t f = fl[((size_t)k * J->ny + j) * b.ntx + tx];
-        weight[((size_t)(k / b.oz) * b.nty + j / b.oy) * b.ntx + tx] += f & 4 ? 4 : f & 0x11 ? 1 : 0;
+        const uint8_t f = fl[r0 + tx];
+        if (!f) continue;
+        w[tx] += f & 4 ? 4 : f & 0x11 ? 1 : 0;
         mixed += f & 4 ? 1 : 0;
+        if (f & ROW_SAMPLE) {
+          smp0 = std::min(smp0, r0 + tx);
+          smp1 = r0 + tx + 1;
+        }
         if (f & 64)  // in every tile whose halo reaches the row
           tiles_of(k, J->nz, J->g.periodic[2], b.oz, 2, b.oz + 4, [&](int tz, int, bool) {
             tiles_of(j, J->ny, J->g.periodic[1], b.oy, 1, b.oy + 3, [&](int ty, int, bool) { ade[((size_t)tz * b.nty + ty) * b.ntx + tx] = 1; });
           });
       }
+    }
   for (int t = 0; t < nt; ++t) order[t] = t;
   for (char c : ade) b.nade += c;
   J->b3_mixed = (int)(8 * mixed / rows);
@@ -1735,17 +1743,17 @@ int setup_block3(fdtd_job *J) {
     if (!J->ade_b && (rc = alloc_dev(J, &J->ade_b, ade_bytes(J)))) return rc;
   }
   // the rows with samples, numbered
-  std::vector<int> seg(rows, 0);
+  std::vector<int> seg(smp1 > smp0 ? smp1 - smp0 : 0, 0);
   int nseg = 0;
-  for (size_t r = 0; r < rows; ++r)
-    if (fl[r] & ROW_SAMPLE) seg[r] = nseg++;
+  for (size_t r = smp0; r < smp1; ++r)
+    if (fl[r] & ROW_SAMPLE) seg[r - smp0] = nseg++;
   if (nseg > 0) {
     J->b3_bytes[3] = (size_t)nseg * 6 * b.ox * sizeof(float);
     if ((rc = alloc_dev(J, (void **)&b.first, J->b3_bytes[3]))) return rc;
     J->b3_bytes[5] = rows * sizeof(int);
     if ((rc = alloc_dev(J, (void **)&b.seg, J->b3_bytes[5]))) return rc;
-    if ((rc = put_dev(J, (void *)b.seg, seg.data(), J->b3_bytes[5]))) return rc;
-    J->h2d += J->b3_bytes[5];
+    if ((rc = put_dev(J, (void *)(b.seg + smp0), seg.data(), seg.size() * sizeof(int)))) return rc;
+    J->h2d += seg.size() * sizeof(int);
   }
   J->block3_ok = true;
   return FDTD_OK;
@@ -1769,6 +1777,7 @@ int setup_fused(fdtd_job *J) {
   if (J->dim != 3 || J->slab_rows > 0 || J->has_tfbox) return FDTD_OK;
   int rc = setup_fused3(J);
   if (rc || J->tile_req > 0) return rc;
+  if (!block3_worth(J)) return FDTD_OK;
   if ((rc = setup_block3(J)) == FDTD_ENOMEM) {
     cudaGetLastError();
     free_block3(J);
@@ -2343,13 +2352,18 @@ int tune_tiles(fdtd_job *J) {
     launch_part<T>(J, p, K2D_CORE, true, J->stream);
     launch_part<T>(J, p, K2D_CORE, false, J->stream);
   };
-  auto time5 = [&](auto run) {
-    for (int w = 0; w < 2; ++w) run();
+  // the time of five runs, from two where they are long and even: of large grids,
+  // and of the 2D block-step kernel's eight steps
+  const bool large = J->ncell >= (J->dim == 3 ? 4000000 : 16000000);
+  auto time5 = [&](auto run, bool few = false) {
+    few |= large;
+    for (int w = 0; w < (few ? 1 : 2); ++w) run();
     cudaEventRecord(a, J->stream);
-    for (int r = 0; r < 5; ++r) run();
+    for (int r = 0; r < (few ? 2 : 5); ++r) run();
     cudaEventRecord(b, J->stream);
     float ms = 0.f;
-    return cudaEventSynchronize(b) == cudaSuccess && cudaEventElapsedTime(&ms, a, b) == cudaSuccess ? ms : 3.0e38f;
+    if (cudaEventSynchronize(b) != cudaSuccess || cudaEventElapsedTime(&ms, a, b) != cudaSuccess) return 3.0e38f;
+    return few ? 2.5f * ms : ms;
   };
   const int last = J->block3_ok ? kBlock3Tile : nshapes - 1;
   for (int c = 0; c <= last; ++c) {
@@ -2370,9 +2384,10 @@ int tune_tiles(fdtd_job *J) {
       }
     }
     p.tile = c;
-    float ms = time5([&] { cores(c); }) / (block ? (float)(J->dim == 2 ? pl.ks : 2) : 1.f);  // of a step
-    // (the first runs of the 3D block-step kernel take a quarter longer than all later ones)
-    if (J->dim == 3 && block) ms = std::min(ms, time5([&] { cores(c); }) / 2.f);
+    // (the first seven runs or so of the 3D block-step kernel take a quarter longer than all later ones)
+    for (int w = 0; w < 6 && J->dim == 3 && block; ++w) cores(c);
+    float ms = time5([&] { cores(c); }, block) / (block ? (float)(J->dim == 2 ? pl.ks : 2) : 1.f);  // of a step
+    if (J->dim == 3 && block) ms = std::min(ms, time5([&] { cores(c); }, block) / 2.f);
     if (block && failed) {  // a kernel that did not run is no candidate
       cudaGetLastError();
       continue;
@@ -3956,7 +3971,8 @@ int fdtd_estimate_bytes(const fdtd_job *J, uint64_t *bytes) {
   if (block3) b += 6 * N * w;
   // the 3D block-step kernel's: the stored PML parts, row flags and segments of
   // the columns of tiles (60 cells), the tiles' order
-  if (block3) {
+  const bool block3w = block3 && block3_worth(J);
+  if (block3w) {
     const uint64_t col = (uint64_t)(nx + 59) / 60;
     b += (J->has_pml ? 6 * N * w : 0) + (uint64_t)ny * nz * col * 5 + col * ((uint64_t)ny / 13 + 1) * ((uint64_t)nz / 8 + 1) * 4;
     for (auto &M : J->mons)
@@ -4007,7 +4023,7 @@ int fdtd_estimate_bytes(const fdtd_job *J, uint64_t *bytes) {
   // and its dispersive cells: a second state, and in up to four tiles a list
   // entry and the scratch state
   if (J->dim == 1 && !J->lean) b += nade * (uint64_t)nf * 3 * w + 32ull * nf * 3 * w;
-  if (block3 && nade > 0) {  // two more states, and the slots over the box
+  if (block3w && nade > 0) {  // two more states, and the slots over the box
     b += 2 * (nade * (uint64_t)nf * 3 * w + 32ull * nf * 3 * w);
     uint64_t box = 4;
     for (int a = 0; a < 3; ++a) box *= (uint64_t)std::max(1, ahi[a] - alo[a] + 1);
