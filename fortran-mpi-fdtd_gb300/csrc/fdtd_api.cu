@@ -254,7 +254,9 @@ struct fdtd_job {
   // stored split-PML parts
   bool block3_ok = false;
   int b3_mixed = 0;  // eighths of its rows with cells of more than the most common material
-  bool lean = false;  // leave out every kernel that needs second sets of buffers
+  // leave out kernels that need second sets of buffers: 1 the block-step kernels,
+  // but for the TMz jobs that have such a set for any kernel of whole steps; 2 all
+  int lean = 0;
   Block3 b3{};
   void *spb3[6] = {};
   size_t b3_bytes[6] = {};  // of the flags, slot map, first step's dispersive state, its sampled rows, order, segments
@@ -645,6 +647,8 @@ size_t ade_bytes(const fdtd_job *J);
 int fused_tile(const fdtd_job *J) { return J->dim == 3 ? 8 : 3; }
 constexpr int kBlock3Tile = 9;
 void free_block3(fdtd_job *J);
+// 2D jobs that count a second set of fields at every footprint but the smallest
+bool block2_always(const fdtd_job *J) { return J->g.layout == FDTD_LAYOUT_2D_TM && J->nx % 4 == 0; }
 // The 3D block-step kernel loses on small grids, whose tiles are few and mostly
 // halo and shell (us a step, block / split: 160^3 123 / 80, 200^3 160 / 143, 128 x
 // 128 x 384 99 / 93; 160 x 160 x 384, 9.8 million cells, 125 / 148), so jobs below
@@ -1765,7 +1769,7 @@ int setup_fused(fdtd_job *J) {
   J->fused_ok = J->block3_ok = false;
   if (getenv("FDTD_NO_FUSED") || J->ncore <= 0) return FDTD_OK;
   if (J->tile_req > 0 && J->tile_req != fused_tile(J) + 1) return FDTD_OK;  // another shape is pinned
-  if (J->lean && J->tile_req == 0) return FDTD_OK;
+  if (J->tile_req == 0 && (J->lean == 2 || (J->lean == 1 && J->dim == 2 && !block2_always(J)))) return FDTD_OK;
   if (J->dim == 2) {
     const int rc = setup_block(J);
     // TMz jobs of 4-cell rows have always had a second set and report its want
@@ -1777,7 +1781,7 @@ int setup_fused(fdtd_job *J) {
   if (J->dim != 3 || J->slab_rows > 0 || J->has_tfbox) return FDTD_OK;
   int rc = setup_fused3(J);
   if (rc || J->tile_req > 0) return rc;
-  if (!block3_worth(J)) return FDTD_OK;
+  if (J->lean || !block3_worth(J)) return FDTD_OK;
   if ((rc = setup_block3(J)) == FDTD_ENOMEM) {
     cudaGetLastError();
     free_block3(J);
@@ -3336,9 +3340,15 @@ int fdtd::pack_run(fdtd::Pack *P, int rings, cudaEvent_t done) {
 }
 
 // =========================================================================
-int fdtd::make_lean(fdtd_job *J, uint64_t *est) {
-  J->lean = true;
-  return fdtd_estimate_bytes(J, est);
+void fdtd::make_lean(fdtd_job *J, int level) { J->lean = level; }
+
+uint64_t fdtd::lean_estimate(fdtd_job *J, int level) {
+  const int own = J->lean;
+  uint64_t est = UINT64_MAX;
+  J->lean = level;
+  fdtd_estimate_bytes(J, &est);
+  J->lean = own;
+  return est;
 }
 
 extern "C" {
@@ -3966,12 +3976,12 @@ int fdtd_estimate_bytes(const fdtd_job *J, uint64_t *bytes) {
   const int nx = J->nx, ny = J->ny, nz = J->nz;
   uint64_t b = N * w * (J->dim == 3 ? 6 : J->dim == 2 ? 3 : 2) + N;  // fields, material ids
   // the fused 3D step kernel's second set of fields (commit may give it back)
-  const bool block3 = J->dim == 3 && w == 4 && J->nx % 4 == 0 && !J->has_tfbox && !J->lean &&
+  const bool block3 = J->dim == 3 && w == 4 && J->nx % 4 == 0 && !J->has_tfbox && J->lean < 2 &&
                       !(J->has_pml && J->pml.mode == FDTD_PML_REFERENCE);
   if (block3) b += 6 * N * w;
   // the 3D block-step kernel's: the stored PML parts, row flags and segments of
   // the columns of tiles (60 cells), the tiles' order
-  const bool block3w = block3 && block3_worth(J);
+  const bool block3w = block3 && !J->lean && block3_worth(J);
   if (block3w) {
     const uint64_t col = (uint64_t)(nx + 59) / 60;
     b += (J->has_pml ? 6 * N * w : 0) + (uint64_t)ny * nz * col * 5 + col * ((uint64_t)ny / 13 + 1) * ((uint64_t)nz / 8 + 1) * 4;
@@ -3981,7 +3991,7 @@ int fdtd_estimate_bytes(const fdtd_job *J, uint64_t *bytes) {
   }
   // the 2D block-step kernel's: the fields and the stored PML part, its tiles
   // (at least 112 x 16 cells, 160 bytes with their flags)
-  const bool block2 = J->dim == 2 && w == 4 && !J->has_tfbox && !J->lean && !(J->has_pml && J->pml.mode == FDTD_PML_REFERENCE);
+  const bool block2 = J->dim == 2 && w == 4 && !J->has_tfbox && J->lean < (block2_always(J) ? 2 : 1) && !(J->has_pml && J->pml.mode == FDTD_PML_REFERENCE);
   if (block2) b += 4 * N * w + ((uint64_t)nx / 112 + 1) * ((uint64_t)ny / 16 + 1) * 160;
   if (J->dim == 1 && !J->lean)  // the 1D block-step kernel's second set and slot map
     b += (J->has_tfsf ? 4 : 2) * N * w + 4 * N + 8ull * (J->pml.npml[1][0] + 2) * w;

@@ -401,9 +401,11 @@ struct DftParams {
   long long stage_row;
   int total_work_blocks;
 };
-// leave the kernels that need second sets of buffers out of an uncommitted job,
-// and estimate again (fdtd_server.cu: a job that would not fit with them)
-int make_lean(fdtd_job *job, uint64_t *est);
+// leave kernels that need second sets of buffers out of an uncommitted job (level
+// 1: the block-step kernels; 2: the fused ones too), and the estimate it then has
+// (fdtd_server.cu: a job that does not fit with them)
+void make_lean(fdtd_job *job, int level);
+uint64_t lean_estimate(fdtd_job *job, int level);
 template <typename T> void launch_dft(const DftParams &d, const T *stage, void *stream);
 // every ring of a line's stage in one launch, for monitors of few samples
 // (dft_rings_fit); d.nslots: the rows of all of them.  Returns the launches.

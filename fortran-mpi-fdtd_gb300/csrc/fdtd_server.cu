@@ -49,6 +49,8 @@ struct Req {
   fdtd_job *job = nullptr;
   int32_t n_steps = 0;
   uint64_t est = 0, bytes = 0;  // footprint: estimate before commit, held after
+  uint64_t est_lean = 0;        // without the block-step kernels' buffers (0: not asked yet)
+  double t_short = 0;           // since when it waits for memory at the head of the queue
   int state = FDTD_REQ_QUEUED;
   int rc = FDTD_OK;
   char err[256] = {};
@@ -106,18 +108,34 @@ void finish(fdtd_server *S, Req *r, int rc, const char *why) {
   S->cv_done.notify_all();
 }
 
+// A job that does not fit beside the active ones waits this long for memory before
+// it runs without what only speeds it up.  (At once, a backlog of short jobs would
+// run every other one at a third to four fifths of its speed; never, a short job
+// could wait for the end of a long one that it used to run beside.)
+constexpr double kLeanWait = 0.1;
+
 // admit queued jobs in order while slots and memory allow (lock held); a
 // commit worker then sets them up
 void admit(fdtd_server *S) {
   while (!S->queue.empty() && (int)S->active.size() + S->committing < S->d.max_active && !S->stop) {
     Req *r = S->queue.front();
-    if (r->est > S->budget) fdtd::make_lean(r->job, &r->est);  // without what only speeds it up
+    for (int level = 1; level <= 2 && r->est > S->budget; ++level) {  // it would never fit
+      fdtd::make_lean(r->job, level);
+      r->est = r->est_lean = fdtd::lean_estimate(r->job, level);
+    }
     if (r->est > S->budget) {
       S->queue.pop_front();
       finish(S, r, FDTD_ENOMEM, "job footprint exceeds the server's HBM budget");
       continue;
     }
-    if (S->held + r->est > S->budget) return;  // wait for memory to be released
+    if (S->held + r->est > S->budget) {  // wait for memory to be released
+      if (r->t_short == 0) r->t_short = now_s();
+      if (now_s() - r->t_short < kLeanWait) return;
+      if (r->est_lean == 0) r->est_lean = fdtd::lean_estimate(r->job, 1);
+      if (r->est_lean >= r->est || S->held + r->est_lean > S->budget) return;
+      fdtd::make_lean(r->job, 1);
+      r->est = r->est_lean;
+    }
     S->queue.pop_front();
     S->held += r->est;
     S->held_max = std::max(S->held_max, S->held);
