@@ -1374,6 +1374,7 @@ int setup_tma(fdtd_job *J) {
 // The 1D block-step kernel takes lines whose slabs continue the main range, with
 // the total-field boundary clear of them and not in a dispersive cell.  (Others
 // stay with the cluster kernel.)
+int setup_line_buffers(fdtd_job *J);
 int setup_line(fdtd_job *J) {
   if (J->dim != 1) return FDTD_OK;
   const int N = J->ny, mlo = J->g.main_lo[1], mhi = J->g.main_hi[1];
@@ -1386,7 +1387,30 @@ int setup_line(fdtd_job *J) {
     for (int c : J->ade_cell_host) if (c == bd) return FDTD_OK;
   }
   if (J->lean) return FDTD_OK;
+  const int rc = setup_line_buffers(J);
+  if (rc != FDTD_ENOMEM) return rc;
+  // no room for its second set: the cluster kernel needs none
+  cudaGetLastError();
+  const size_t bytes = (size_t)N * J->esz, slab = (size_t)(J->pml.npml[1][0] + 2) * J->esz;
+  auto give = [&](void *&p, size_t n) {
+    free_dev(J, p, n);
+    p = nullptr;
+  };
+  for (void *&p : J->lineB) give(p, bytes);
+  for (int l = 0; l < 2; ++l)
+    for (int s = 0; s < 2; ++s) {
+      give(J->lineB_lex[l][s], slab);
+      give(J->lineB_lhz[l][s], slab);
+    }
+  free_dev(J, J->d_line_slot, N * sizeof(int));
+  J->d_line_slot = nullptr;
+  give(J->ade_b, ade_bytes(J));
+  return FDTD_OK;
+}
+
+int setup_line_buffers(fdtd_job *J) {
   int rc;
+  const int N = J->ny;
   const size_t w = J->esz;
   for (int q = 0; q < (J->has_tfsf ? 4 : 2); ++q)
     if ((rc = alloc_dev(J, &J->lineB[q], N * w))) return rc;

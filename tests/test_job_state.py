@@ -190,3 +190,36 @@ def test_failed_pack_capture_leaves_the_members(gpu, monkeypatch, after):
     finally:
         gpu.fail_launch_after(-1)
         S.close()
+
+
+def test_line_without_room_for_a_second_set(gpu):
+    """A 1D job whose second set of buffers cannot be had runs in the kernel that
+    needs none, with the same results; other allocations of set-up still fail it."""
+    spec, _ = problems.config_1d_gold(precision=abi.F64)
+    ref = gpu.Job(spec)
+    full = ref.device_bytes()
+    ref.step(1, 700)
+    want = state_of(ref, (abi.EX, abi.HZ))
+    ref.close()
+    refused = without = 0
+    try:
+        for k in range(200):
+            gpu.fail_alloc_after(k)
+            try:
+                J = gpu.Job(spec)
+            except gpu.FdtdError as e:
+                assert e.code == abi.FDTD_ENOMEM
+                refused += 1
+                continue
+            gpu.fail_alloc_after(-1)
+            if J.device_bytes() == full:
+                J.close()
+                break
+            without += 1
+            J.step(1, 700)
+            for a, b in zip(state_of(J, (abi.EX, abi.HZ)), want):
+                np.testing.assert_array_equal(a, b)
+            J.close()
+    finally:
+        gpu.fail_alloc_after(-1)
+    assert refused > 10 and without >= 4
