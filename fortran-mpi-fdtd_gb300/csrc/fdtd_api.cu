@@ -3070,7 +3070,13 @@ template <typename T>
 static int get_field_impl(fdtd_job *J, int comp, double *host) {
   if (comp < 0 || comp > 7 || !J->F[comp]) return set_err(FDTD_EINVAL, "component %d not in this layout", comp);
   const long long cnt = field_elems(J, comp);
-  const void *from = J->pp && comp < 6 ? J->Fb[comp] : J->F[comp];  // the current set
+  // From the current set; a job that replays graphs needs the canonical one next,
+  // and the copies cost least here, where the host waits anyway (611 x 407, 200
+  // steps and a frame: 846 us, 860 with the copies before the next replay).  A job
+  // stepped one by one with a frame each (256^2) takes 44 us, 66 with the copies.
+  if (J->graph_exec)
+    if (const int rc = fused_settle(J)) return rc;
+  const void *from = J->pp && comp < 6 ? J->Fb[comp] : J->F[comp];
   std::vector<T> tmp((size_t)cnt);
   CK(cudaMemcpyAsync(tmp.data(), from, (size_t)cnt * sizeof(T), cudaMemcpyDeviceToHost, J->stream));
   CK(cudaStreamSynchronize(J->stream));
