@@ -281,22 +281,21 @@ struct fdtd_job {
   long long launches = 0;
   cudaStream_t own_stream = nullptr;
   uint64_t h2d = 0, d2h = 0;
-  // 2D work split (core box + edge unit list) and the streams that run the
-  // parts of a half step as parallel branches of the job's stream
+  // 2D and 3D work split (core box + edge unit list) and the stream that runs the
+  // second part of a half step, or of a block-step launch, beside the first
   int vec = 1, cv0 = 0, cw = 0, cy0 = 0, ncore = 0, nedge = 0;
   int ch = 0, cz0 = 0, cd = 0;  // 3D: core box rows and planes
   int tile_req = 0, tile = 1;    // core block shape: requested (0: tune) and used
   int split_tile = 1;            // of the split kernels beside a block-step kernel
   int block_min = 1;             // least steps of a 2D block-step launch from the canonical field set
   int *d_edge = nullptr;
-  cudaStream_t side[2] = {};
-  cudaEvent_t ev_fork = nullptr, ev_join[2] = {};
+  cudaStream_t side = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   // programmatic events of the last two core kernels; prog_prev indexes
-  // the one the next half step's side kernels may wait on (-1: none, after
+  // the one the next half step's side kernel may wait on (-1: none, after
   // any other kernel on the job's stream)
   cudaEvent_t ev_prog[2] = {};
   int prog_prev = -1;
-  bool join_rec[2] = {false, false};
 };
 
 namespace {
@@ -544,13 +543,11 @@ int upload_prof(fdtd_job *J, const Prof &P, void **f1, void **f2, void **g1, voi
 }
 
 // ---- commit ------------------------------------------------------------
-// side streams and events that fork a half step's parts off the job's stream
+// side stream and events that fork a half step's parts off the job's stream
 int make_branches(fdtd_job *J) {
-  for (int q = 0; q < 2; ++q) {
-    CK(cudaStreamCreateWithFlags(&J->side[q], cudaStreamNonBlocking));
-    CK(cudaEventCreateWithFlags(&J->ev_join[q], cudaEventDisableTiming));
-    CK(cudaEventCreateWithFlags(&J->ev_prog[q], cudaEventDisableTiming));
-  }
+  CK(cudaStreamCreateWithFlags(&J->side, cudaStreamNonBlocking));
+  CK(cudaEventCreateWithFlags(&J->ev_join, cudaEventDisableTiming));
+  for (int q = 0; q < 2; ++q) CK(cudaEventCreateWithFlags(&J->ev_prog[q], cudaEventDisableTiming));
   CK(cudaEventCreateWithFlags(&J->ev_fork, cudaEventDisableTiming));
   CK(cudaStreamCreateWithFlags(&J->fold_stream, cudaStreamNonBlocking));
   CK(cudaEventCreateWithFlags(&J->ev_ffork, cudaEventDisableTiming));
@@ -1681,9 +1678,10 @@ int setup_fused3(fdtd_job *J) {
   return FDTD_OK;
 }
 
-// The 3D block-step kernel takes any FP32 grid of even row length without
-// reference slabs or a TFSF box (those update fields in place), and materials
-// whose z update does not read the x update's current.
+// The 3D block-step kernel takes FP32 grids whose rows are 4-cell vectors (its own
+// pairs of cells need even rows) without reference slabs or a TFSF box (those
+// update fields in place), and materials whose z update does not read the x
+// update's current.
 int setup_block3(fdtd_job *J) {
   if (J->esz != 4 || J->vec != 4 || J->nz < 2 || (unsigned long long)J->ncell >= 1ull << 30) return FDTD_OK;
   const AdeCoef<float> *ac = reinterpret_cast<const AdeCoef<float> *>(J->ac_host.data());
@@ -2116,8 +2114,9 @@ enum { ST_E = 1, ST_H = 2, ST_SAMPLE = 4 };
 // The parts of one half step write disjoint cells and read only the other
 // half's fields, so they run as parallel branches of the job's stream
 // (forked and joined with events; a stream capture records them as parallel
-// graph nodes).  2D: core, edge and ADE launches; 3D: core and the general
-// launch (tiles with non-core cells, reference slabs, ADE cells).  Profiled
+// graph nodes).  2D: the core launch and one of the edge units and dispersive
+// cells; 3D: core and the general launch (tiles with non-core cells, reference
+// slabs, ADE cells).  Profiled
 // runs launch them one after another so that each part's events time that
 // part alone.
 template <typename T>
@@ -2128,60 +2127,45 @@ int launch_part(const fdtd_job *J, const StepParams<T> &p, int part, bool e_half
 }
 
 template <typename T>
-int run_parts(fdtd_job *J, const StepParams<T> &p, const bool (&want)[3], bool e_half, bool graph) {
-  static const int kind[3] = {-1, FDTD_KERNEL_EDGE, FDTD_KERNEL_ADE};
+int run_parts(fdtd_job *J, const StepParams<T> &p, const bool (&want)[2], bool e_half, bool graph) {
   const int general = J->dim == 2 ? p.nedge + (e_half ? p.nade : 0) : p.ntile_blocks + p.nslab_blocks + (e_half ? p.nade_blocks : 0);
-  const int units[3] = {p.ncore, general, J->dim == 2 && e_half ? p.nade : 0};
-  int use[3], nuse = 0;
-  for (int q = 0; q < 3; ++q)
-    if (want[q] && units[q] > 0) use[nuse++] = q;
-  const bool par = !J->prof && nuse > 1;
-  // The side kernels of this half step wait on the previous core
-  // kernel's programmatic event rather than on its completion, so that they
-  // are ready together with this half's core kernel (they wait for the
-  // previous core kernel in their own pdl_wait), and fully on the side
-  // streams' previous kernels; otherwise they fork off the job's stream.
-  const bool chain = par && use[0] == K2D_CORE;
-  const bool prog = chain && J->prog_prev >= 0;
-  cudaStream_t st[3] = {J->stream, J->stream, J->stream};
-  if (par) {
-    if (!prog) CK(cudaEventRecord(J->ev_fork, J->stream));
-    for (int b = 1; b < nuse; ++b) {
-      st[b] = J->side[b - 1];
-      if (prog) {
-        CK(cudaStreamWaitEvent(st[b], J->ev_prog[J->prog_prev], 0));
-        for (int c = 0; c < 2; ++c)
-          if (c != b - 1 && J->join_rec[c]) CK(cudaStreamWaitEvent(st[b], J->ev_join[c], 0));
-      } else {
-        CK(cudaStreamWaitEvent(st[b], J->ev_fork, 0));
-      }
-    }
+  const bool core = want[K2D_CORE] && p.ncore > 0, edge = want[K2D_EDGE] && general > 0;
+  const bool par = !J->prof && core && edge;
+  // The side kernel of this half step waits on the previous core kernel's
+  // programmatic event rather than on its completion, so that it is ready
+  // together with this half's core kernel (it waits for the previous core
+  // kernel in its own pdl_wait), and fully on the side stream's previous
+  // kernel; otherwise it forks off the job's stream.
+  const bool prog = par && J->prog_prev >= 0;
+  cudaStream_t side = par ? J->side : J->stream;
+  if (prog) {
+    CK(cudaStreamWaitEvent(side, J->ev_prog[J->prog_prev], 0));
+  } else if (par) {
+    CK(cudaEventRecord(J->ev_fork, J->stream));
+    CK(cudaStreamWaitEvent(side, J->ev_fork, 0));
   }
   const int cur = J->prog_prev == 0 ? 1 : 0;
-  for (int b = 0; b < nuse; ++b) {
-    const int q = use[b];
-    const int k = q == K2D_CORE ? (e_half ? FDTD_KERNEL_E : FDTD_KERNEL_H) : kind[q];
-    if (!graph) ev_record(J, k, true);
-    J->launches += launch_part<T>(J, p, q, e_half, st[b], chain && q == K2D_CORE ? J->ev_prog[cur] : nullptr);
-    if (!graph) ev_record(J, k, false);
-  }
+  auto run = [&](int part, int kind, cudaStream_t s, cudaEvent_t ev) {
+    if (!graph) ev_record(J, kind, true);
+    J->launches += launch_part<T>(J, p, part, e_half, s, ev);
+    if (!graph) ev_record(J, kind, false);
+  };
+  if (core) run(K2D_CORE, e_half ? FDTD_KERNEL_E : FDTD_KERNEL_H, J->stream, par ? J->ev_prog[cur] : nullptr);
+  if (edge) run(K2D_EDGE, FDTD_KERNEL_EDGE, side, nullptr);
   CK(cudaGetLastError());
   if (par) {
-    for (int b = 1; b < nuse; ++b) {
-      CK(cudaEventRecord(J->ev_join[b - 1], st[b]));
-      J->join_rec[b - 1] = true;
-      CK(cudaStreamWaitEvent(J->stream, J->ev_join[b - 1], 0));
-    }
+    CK(cudaEventRecord(J->ev_join, side));
+    CK(cudaStreamWaitEvent(J->stream, J->ev_join, 0));
   }
-  J->prog_prev = chain ? cur : -1;
+  J->prog_prev = par ? cur : -1;
   return FDTD_OK;
 }
 
-// Commit-time tuner of the core kernels' block shape.  Each candidate runs a
-// few E and H core launches on the job's own grid, whose fields are still
-// zero -- a core update of zero fields writes back the zeros it read -- and
-// the fastest is kept.  The choice is cached per kind of grid (dimension,
-// layout, precision, vector width, log2 of the core cells).
+// Commit-time tuner of the core kernels' block shape and of the kernels that take
+// whole steps.  Each candidate runs a few times on the job's own grid, whose
+// fields are still zero -- an update of zero fields writes back the zeros it read
+// -- and the fastest is kept.  The choice is cached per kind of grid (the key in
+// tune_tiles).
 std::mutex g_tune_mu;
 std::map<std::array<long long, 2>, int> g_tune;
 
@@ -2219,13 +2203,13 @@ void block3_buffers(const fdtd_job *J, StepParams<float> &p, Block3 &b, int from
 // stream.  Returns the kernels launched, -1 on failure.
 int launch_blocks(fdtd_job *J, const StepParams<float> &p, const BlockPlan &pl) {
   const bool both = pl.ngen > 0 && pl.ngen < pl.ntiles && !J->prof;
-  cudaStream_t side = both ? J->side[0] : J->stream;
+  cudaStream_t side = both ? J->side : J->stream;
   cudaError_t e = fails_now(g_fail_launch) ? cudaErrorLaunchFailure : cudaSuccess;
   if (both && e == cudaSuccess && (e = cudaEventRecord(J->ev_fork, J->stream)) == cudaSuccess)
     e = cudaStreamWaitEvent(side, J->ev_fork, 0);
   const int n0 = e == cudaSuccess ? launch_step2d_block(p, pl, true, J->stream) : -1;
   const int n1 = n0 >= 0 ? launch_step2d_block(p, pl, false, side) : -1;
-  if (both && n1 >= 0 && (e = cudaEventRecord(J->ev_join[0], side)) == cudaSuccess) e = cudaStreamWaitEvent(J->stream, J->ev_join[0], 0);
+  if (both && n1 >= 0 && (e = cudaEventRecord(J->ev_join, side)) == cudaSuccess) e = cudaStreamWaitEvent(J->stream, J->ev_join, 0);
   if (n1 < 0 || e != cudaSuccess) {
     set_err(FDTD_ECUDA, "2D block-step launch: %s", cudaGetErrorString(e != cudaSuccess ? e : cudaGetLastError()));
     return -1;
@@ -2237,13 +2221,13 @@ int launch_blocks(fdtd_job *J, const StepParams<float> &p, const BlockPlan &pl) 
 // without that code and its registers.
 int launch_blocks3(fdtd_job *J, const StepParams<float> &p, const Block3 &b, int k) {
   const bool both = b.nade > 0 && b.nade < b.ntx * b.nty * b.ntz && !J->prof;
-  cudaStream_t side = both ? J->side[0] : J->stream;
+  cudaStream_t side = both ? J->side : J->stream;
   cudaError_t e = fails_now(g_fail_launch) ? cudaErrorLaunchFailure : cudaSuccess;
   if (both && e == cudaSuccess && (e = cudaEventRecord(J->ev_fork, J->stream)) == cudaSuccess)
     e = cudaStreamWaitEvent(side, J->ev_fork, 0);
   const int n0 = e == cudaSuccess ? launch_step3d_block(p, b, k, true, J->stream) : -1;
   const int n1 = n0 >= 0 ? launch_step3d_block(p, b, k, false, side) : -1;
-  if (both && n1 >= 0 && (e = cudaEventRecord(J->ev_join[0], side)) == cudaSuccess) e = cudaStreamWaitEvent(J->stream, J->ev_join[0], 0);
+  if (both && n1 >= 0 && (e = cudaEventRecord(J->ev_join, side)) == cudaSuccess) e = cudaStreamWaitEvent(J->stream, J->ev_join, 0);
   if (n1 < 0 || e != cudaSuccess) {
     set_err(FDTD_ECUDA, "3D block-step launch: %s", cudaGetErrorString(e != cudaSuccess ? e : cudaGetLastError()));
     return -1;
@@ -2319,17 +2303,14 @@ int tune_tiles(fdtd_job *J) {
   float best = 3.0e38f, best_split = 3.0e38f;
   int choice = 1;
   // 3D: also the z-marching kernels and, where set up, the TMA-staged cores
-  // and the fused step kernel (one launch in place of an E and an H core).
-  // 2D: also the fused step kernel, against the E and H cores alone (in a
-  // step the edge and dispersive-cell kernels run beside the cores, and
-  // their work is a small part of a grid large enough for the fused kernel)
+  // and the fused step kernel (one launch in place of an E and an H core)
   const int nshapes = J->dim == 3 ? (J->fused_ok ? 9 : J->tma_ok ? (J->tma.h_ok ? 8 : 7) : 6) : J->fused_ok ? 4 : 3;
   // The block-step kernels take whole steps, so they are timed against the whole
   // step of the best other shape: cores, edge and dispersive cells
   BlockPlan pl{};
   if (J->dim == 2 && J->fused_ok) block_plan(J, pl);
   auto split_step = [&] {
-    const bool parts[3] = {true, true, false};
+    const bool parts[2] = {true, true};
     p.roles = ROLE_MAIN | ROLE_PML | ROLE_ADE;
     p.tile = choice;
     if constexpr (sizeof(T) == 4) {
@@ -2472,7 +2453,7 @@ int half_e(fdtd_job *J, int n, int roles, int slot = 0, bool graph = false) {
   p.n = n;
   p.slot = slot;
   ring_params(J, p, graph);
-  const bool parts[3] = {(roles & ROLE_MAIN) != 0, (roles & (ROLE_MAIN | ROLE_PML | ROLE_ADE)) != 0, false};
+  const bool parts[2] = {(roles & ROLE_MAIN) != 0, (roles & (ROLE_MAIN | ROLE_PML | ROLE_ADE)) != 0};
   int rc = run_parts<T>(J, p, parts, true, graph);
   if (!rc && J->has_tfbox && (roles & ROLE_MAIN)) rc = tfsf_part<T>(J, p, true, graph);
   return rc;
@@ -2487,7 +2468,7 @@ int half_h(fdtd_job *J, int n, int roles, bool gather, int slot = -1, bool graph
   p.gather = gather ? 1 : 0;
   p.slot = slot >= 0 ? slot : J->stage_fill;
   ring_params(J, p, graph);
-  const bool parts[3] = {(roles & ROLE_MAIN) != 0, (roles & (ROLE_MAIN | ROLE_PML)) != 0, false};
+  const bool parts[2] = {(roles & ROLE_MAIN) != 0, (roles & (ROLE_MAIN | ROLE_PML)) != 0};
   int rc = run_parts<T>(J, p, parts, false, graph);
   if (!rc && J->has_tfbox && (roles & ROLE_MAIN)) rc = tfsf_part<T>(J, p, false, graph);
   return rc;
@@ -3457,10 +3438,10 @@ int fdtd_destroy(fdtd_job *J) {
   for (auto &e : J->pending) { cudaEventDestroy(e.a); if (e.b) cudaEventDestroy(e.b); }
   for (auto e : J->ev_pool) cudaEventDestroy(e);
   for (int q = 0; q < 2; ++q) {
-    if (J->side[q]) cudaStreamDestroy(J->side[q]);
-    if (J->ev_join[q]) cudaEventDestroy(J->ev_join[q]);
     if (J->ev_prog[q]) cudaEventDestroy(J->ev_prog[q]);
   }
+  if (J->side) cudaStreamDestroy(J->side);
+  if (J->ev_join) cudaEventDestroy(J->ev_join);
   if (J->ev_fork) cudaEventDestroy(J->ev_fork);
   for (auto &c : J->src_call)
     if (c.done) cudaEventDestroy(c.done);
