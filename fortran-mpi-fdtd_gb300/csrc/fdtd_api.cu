@@ -243,6 +243,7 @@ struct fdtd_job {
   // dispersive cells, and the scratch for state beyond shared memory
   struct BlockTables {
     int shape = 0, ks = 0, max_ade = 0, ntiles = 0, ngen = 0, scr_stride = 0;
+    long long dense = 0;  // most samples a step of a tile with more than kBlockRows sampled rows
     BlockGeom g{};
     Tile2 *tiles = nullptr;
     uint32_t *sflags[2] = {};  // of plain and general tiles
@@ -1543,6 +1544,17 @@ int setup_block(fdtd_job *J) {
     for (int w = 0; w < sh.NA; ++w) f |= sf[(size_t)t * sh.NA + w] & 0xffu;
     general[t] = f != 0;
     all[t].smp = f & SF_SMP ? 1 : 0;
+    // samples of a tile that takes them without shared memory
+    int srows = 0;
+    for (int y = g.hy; y < g.hy + g.oy; ++y) srows += sf[(size_t)t * sh.NA + y / sh.RA] >> (16 + y % sh.RA) & 1u;
+    if (srows > kBlockRows) {
+      long long cells = 0;
+      const int tx0 = all[t].tx * g.ox, ty0 = all[t].y0;
+      for (const Monitor &m : J->mon_dev)
+        cells += (long long)m.ncomp * std::max(0, std::min(tx0 + g.ox - 1, m.hi[0]) - std::max(tx0, m.lo[0]) + 1) *
+                 std::max(0, std::min(ty0 + g.oy - 1, m.hi[1]) - std::max(ty0, m.lo[1]) + 1);
+      B.dense = std::max(B.dense, cells);
+    }
   }
   // f(first cell, cells, tile, place of the first in the tile, from which to which
   // of them the tile owns) of the dispersive cells, a stretch of a row at a time;
@@ -2270,6 +2282,7 @@ int tune_tiles(fdtd_job *J) {
   int lade = 0;
   for (long long c = J->nade; lade < 15 && c < J->ncore; c *= 2, ++lade)
     if (c == 0) { lade = 15; break; }
+  // and the most samples of a tile that stages them itself (its powers of two),
   // and how well the grid fills the 3D block-step kernel's tiles (sixteenths of the
   // cells of its rounds: 320 x 320 x 200 411 us a step there and 315 split, 320 x
   // 240 x 300, of as many cells, 279 and 353)
@@ -2280,10 +2293,12 @@ int tune_tiles(fdtd_job *J) {
     fill = 16ll * J->ncell / (waves * (b.oz + 6) * J->num_sms * b.ox * b.oy);
   }
   const long long mixed = J->dim == 2 && J->fused_ok ? 8ll * J->blk.ngen / std::max(1, J->blk.ntiles) : J->b3_mixed;
+  int dense = 0;
+  for (long long c = J->blk.dense; c > 0; c >>= 1) ++dense;
   const std::array<long long, 2> key = {
       ((((((long long)J->dim * 8 + J->g.layout) * 4 + J->g.precision) * 8 + J->vec) * 64 + lg) * 16 + lade) * 8 +
           (J->fused_ok ? 4 : 0) + (J->tma_ok ? 2 : 0) + (J->tma_ok && J->tma.h_ok ? 1 : 0),
-      (((J->ade_kind + 1ll) * 16 + mixed) * 32 + fill) * 4 + (J->ac_host.size() > sizeof(AdeCoef<T>) ? 2 : 0) + (J->block3_ok ? 1 : 0)};
+      ((((J->ade_kind + 1ll) * 16 + mixed) * 32 + fill) * 32 + dense) * 4 + (J->ac_host.size() > sizeof(AdeCoef<T>) ? 2 : 0) + (J->block3_ok ? 1 : 0)};
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     auto it = g_tune.find(key);
@@ -2306,8 +2321,11 @@ int tune_tiles(fdtd_job *J) {
   // and the fused step kernel (one launch in place of an E and an H core)
   const int nshapes = J->dim == 3 ? (J->fused_ok ? 9 : J->tma_ok ? (J->tma.h_ok ? 8 : 7) : 6) : J->fused_ok ? 4 : 3;
   // The block-step kernels take whole steps, so they are timed against the whole
-  // step of the best other shape: cores, edge and dispersive cells
+  // step of the best other shape: cores, edge and dispersive cells, in 2D with the
+  // samples (a monitor over the whole of 2048^2: 78 us a step in the block-step
+  // kernel when it took them cell by cell, 51 split)
   BlockPlan pl{};
+  p.gather = J->dim == 2 && J->gather_fused;
   if (J->dim == 2 && J->fused_ok) block_plan(J, pl);
   auto split_step = [&] {
     const bool parts[2] = {true, true};

@@ -314,6 +314,7 @@ struct BlockShape {
 };
 constexpr int kBlockShapes = 2;
 constexpr int kBlockSteps = 8;  // most steps of a launch
+constexpr int kBlockRows = 2;   // rows of a tile whose samples are staged through shared memory
 BlockShape block_shape(int shape);
 // bytes of dynamic shared memory (and the plan's offsets) for tiles with at
 // most max_ade dispersive cells; sets cap

@@ -38,8 +38,6 @@ namespace {
 
 typedef float T;
 
-constexpr int kBlockRows = 2;  // rows of a tile whose samples are staged through shared memory
-
 template <int M>
 struct Mode {
   static constexpr int value = M;
@@ -50,15 +48,18 @@ __device__ __forceinline__ int wrap_i(int i, int n) {
   return i < 0 ? i + n : i;
 }
 
-// whether the cells lo..hi of row j hold a sample (mons: monitors count)
-__device__ __forceinline__ bool row_sampled(const StepParams<T> &p, int j, int lo, int hi, bool mons = true) {
-  for (int q = 0; mons && q < p.nmon; ++q) {
-    const Monitor &m = p.mon[q];
-    if (j >= m.lo[1] && j <= m.hi[1] && hi >= m.lo[0] && lo <= m.hi[0]) return true;
-  }
+// whether the cells lo..hi of row j hold a probe, or a sample of any kind
+__device__ __forceinline__ bool row_probed(const StepParams<T> &p, int j, int lo, int hi) {
   for (int q = 0; q < p.nprobe; ++q)
     if (p.probe[q].cell[1] == j && p.probe[q].cell[0] >= lo && p.probe[q].cell[0] <= hi) return true;
   return false;
+}
+__device__ __forceinline__ bool row_sampled(const StepParams<T> &p, int j, int lo, int hi) {
+  for (int q = 0; q < p.nmon; ++q) {
+    const Monitor &m = p.mon[q];
+    if (j >= m.lo[1] && j <= m.hi[1] && hi >= m.lo[0] && lo <= m.hi[0]) return true;
+  }
+  return row_probed(p, j, lo, hi);
 }
 
 // Flags (SF_*) of the warp strips of the plan's tiles, from the material ids and
@@ -336,7 +337,7 @@ __device__ __forceinline__ void block_tile(const StepParams<T> &p, const BlockPl
   for (int t = threadIdx.x; GEN && t < pl.ks * p.nsrc; t += NT)
     srcv[t] = T(p.srcval_tab[(long long)(n0 - 1) * p.nsrc + t]);
   // the owned rows with samples: their number in the tile, in the order of
-  // warps; more than kBlockRows of them are staged cell by cell
+  // warps; more than kBlockRows of them go straight to the stage ring
   int srow0 = 0, nsrow = 0;
   if (GEN && tl.smp) {
     if (lane == 0) rowcnt[w] = __popc(grow);
@@ -348,16 +349,15 @@ __device__ __forceinline__ void block_tile(const StepParams<T> &p, const BlockPl
     if (nsrow <= kBlockRows && lane == 0)
       for (unsigned m = grow, k = srow0; m; m &= m - 1, ++k) rowj[k] = yr + __ffs(m) - 1;
   }
-  // the thread's cells that are taken one by one: a line along y is one cell of
-  // four in a row, and the loop over them is what a tile with such a line waits for
-  // (bits of grow above its rows': the loop has no register to spare)
-  if (GEN && grow && (nsrow > kBlockRows || p.nprobe > 0))
+  // the thread's cells with a probe (bits of grow above its rows': the loop over
+  // the steps has no register to spare)
+  if (GEN && grow && p.nprobe > 0)
 #pragma unroll 1
     for (unsigned m = grow; m; m &= m - 1) {
       const int rr = __ffs(m) - 1;
 #pragma unroll 1
       for (int q = 0; q < V; ++q)
-        if (((xow >> q) & 1u) && row_sampled(p, yr + rr, xr + q, xr + q, nsrow > kBlockRows)) grow |= 1u << (R + rr * V + q);
+        if (((xow >> q) & 1u) && row_probed(p, yr + rr, xr + q, xr + q)) grow |= 1u << (R + rr * V + q);
     }
   if (GEN && KIND != MK_GOLD && adem) {  // their E before the first step
 #pragma unroll
@@ -665,6 +665,37 @@ __device__ __forceinline__ void block_tile(const StepParams<T> &p, const BlockPl
             vst<T, V>(d + 2 * W, c[r]);
             d += 3 * W;
           }
+      } else {
+        // many rows (a line along y, an area): straight to the stage ring, every
+        // cell of a monitor's component by a store of its own register
+        T *const stg = stage_ring(p) + (long long)(p.slot + s) * p.stage_row;
+        const int x0 = tl.tx * pl.g.ox, x1 = min(x0 + pl.g.ox, nx) - 1;
+#pragma unroll 1
+        for (int t = 0; t < p.nmon; ++t) {
+          const Monitor &mo = p.mon[t];
+          if (x1 < mo.lo[0] || x0 > mo.hi[0] || yr + R - 1 < mo.lo[1] || yr > mo.hi[1]) continue;
+          const int wx = mo.hi[0] - mo.lo[0] + 1;
+#pragma unroll 1
+          for (int u = 0; u < mo.ncomp; ++u) {
+            const int cc = mo.comps[u];
+            T *const to = stg + mo.base + (long long)u * mo.ncell + (xr - mo.lo[0]);
+            auto put = [&](auto value) __attribute__((always_inline)) {
+#pragma unroll
+              for (int r = 0; r < R; ++r) {
+                const int j = yr + r;
+                if (!((grow >> r) & 1u) || j < mo.lo[1] || j > mo.hi[1]) continue;
+                T *const row = to + (long long)wx * (j - mo.lo[1]);
+#pragma unroll
+                for (int q = 0; q < V; ++q)
+                  if (((xow >> q) & 1u) && xr + q >= mo.lo[0] && xr + q <= mo.hi[0]) row[q] = value(r, q);
+              }
+            };
+            if (cc == (TM ? 2 : 0)) put([&](int r, int q) { return a[r][q]; });
+            else if (cc == (TM ? 3 : 1)) put([&](int r, int q) { return b[r][q]; });
+            else if (cc == (TM ? 4 : 5)) put([&](int r, int q) { return c[r][q]; });
+            else put([&](int, int) { return T(0); });
+          }
+        }
       }
 #pragma unroll 1
       for (unsigned m = __reduce_or_sync(0xffffffffu, grow >> R); m; m &= m - 1) {
@@ -681,7 +712,7 @@ __device__ __forceinline__ void block_tile(const StepParams<T> &p, const BlockPl
               vc = c[r][u];
             }
         const T vals[6] = {TM ? T(0) : va, TM ? T(0) : vb, TM ? va : T(0), TM ? vb : T(0), TM ? vc : T(0), TM ? T(0) : vc};
-        gather_cell<T>(p, n, xr + at % V, yr + at / V, 0, vals, p.slot + s, nsrow > kBlockRows);
+        gather_cell<T>(p, n, xr + at % V, yr + at / V, 0, vals, p.slot + s, false);
       }
     }
   }

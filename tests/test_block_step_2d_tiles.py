@@ -70,6 +70,7 @@ def test_columns_of_samples_and_sources(gpu, monkeypatch, te, nx, ny, kw):  # no
         spec.add_monitor((x, 3, 0), (x, ny - 4, 0), (e, h), om)
         spec.add_probe((x, ny // 2, 0), (e, h))
     spec.add_monitor((100, 20, 0), (130, 40, 0), (h, e), om)
+    spec.add_monitor((0, 0, 0), (nx - 1, ny - 1, 0), (e, abi.EY if te else abi.HY, h), om[:1])
     for x in (lo for lo in (spec.main_lo[0], 105, 112) if lo <= spec.main_hi[0]):
         spec.sources.append(dict(component=e, lo=(x, 5, 0), hi=(x, ny - 6, 0), amp=0.3, t0=1e-16, st=2e-16, w0=3e15))
     calls = (3, 8, 64, 17, 31)
