@@ -255,6 +255,8 @@ struct fdtd_job {
   // stored split-PML parts
   bool block3_ok = false;
   int b3_mixed = 0;  // eighths of its rows with cells of more than the most common material
+  int b3_slow = 0;   // most eighths of a tile's planes with a row that takes the general round
+  int b3_src = 0;    // halvings of its rows down to those with sources, up to 15
   // leave out kernels that need second sets of buffers: 1 the block-step kernels,
   // but for the TMz jobs that have such a set for any kernel of whole steps; 2 all
   int lean = 0;
@@ -1713,6 +1715,7 @@ int setup_block3(fdtd_job *J) {
   {
     StepParams<float> p;
     fill_common<float>(J, p);
+    set_sources<float>(J, p);
     launch_row_flags3(p, b, (uint8_t *)b.flags, J->stream);
     CK(cudaGetLastError());
   }
@@ -1724,17 +1727,24 @@ int setup_block3(fdtd_job *J) {
   std::vector<int> order((size_t)nt);
   std::vector<long long> weight((size_t)nt, 0);
   std::vector<char> ade((size_t)nt, 0);
-  size_t mixed = 0;
+  size_t mixed = 0, driven = 0;
+  std::vector<int> slow((size_t)nt, 0), seen((size_t)nt, -1);  // planes of a tile with a slow row; the last of them
   size_t smp0 = rows, smp1 = 0;  // from the first to past the last row with samples
   for (int k = 0; k < J->nz; ++k)
     for (int j = 0; j < J->ny; ++j) {
       const size_t r0 = ((size_t)k * J->ny + j) * b.ntx;
-      long long *const w = weight.data() + ((size_t)(k / b.oz) * b.nty + j / b.oy) * b.ntx;
+      const size_t t0 = ((size_t)(k / b.oz) * b.nty + j / b.oy) * b.ntx;
+      long long *const w = weight.data() + t0;
       for (int tx = 0; tx < b.ntx; ++tx) {
         const uint8_t f = fl[r0 + tx];
         if (!f) continue;
         w[tx] += f & 4 ? 4 : f & 0x11 ? 1 : 0;
         mixed += f & 4 ? 1 : 0;
+        driven += f & ROW_SRC ? 1 : 0;
+        if (f & (4 | 32 | ROW_SRC) && seen[t0 + tx] != k) {  // materials, z shells, sources
+          seen[t0 + tx] = k;
+          ++slow[t0 + tx];
+        }
         if (f & ROW_SAMPLE) {
           smp0 = std::min(smp0, r0 + tx);
           smp1 = r0 + tx + 1;
@@ -1748,6 +1758,8 @@ int setup_block3(fdtd_job *J) {
   for (int t = 0; t < nt; ++t) order[t] = t;
   for (char c : ade) b.nade += c;
   J->b3_mixed = (int)(8 * mixed / rows);
+  for (J->b3_src = 0; J->b3_src < 15 && (driven << J->b3_src) < rows;) ++J->b3_src;
+  J->b3_slow = 8 * *std::max_element(slow.begin(), slow.end()) / b.oz;
   std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
     return ade[x] != ade[y] ? ade[x] > ade[y] : weight[x] / 64 > weight[y] / 64;
   });
@@ -2282,7 +2294,9 @@ int tune_tiles(fdtd_job *J) {
   int lade = 0;
   for (long long c = J->nade; lade < 15 && c < J->ncore; c *= 2, ++lade)
     if (c == 0) { lade = 15; break; }
-  // and the most samples of a tile that stages them itself (its powers of two),
+  // and in 3D the share of rows with sources (halvings), the longest run of general rounds of a tile (a line of sources along
+  // z, one row of a plane, 400^3: 1310 us a step in the block-step kernel and 797
+  // split, without it 638 and 792), the most samples of a tile that stages them itself (its powers of two),
   // and how well the grid fills the 3D block-step kernel's tiles (sixteenths of the
   // cells of its rounds: 320 x 320 x 200 411 us a step there and 315 split, 320 x
   // 240 x 300, of as many cells, 279 and 353)
@@ -2293,12 +2307,12 @@ int tune_tiles(fdtd_job *J) {
     fill = 16ll * J->ncell / (waves * (b.oz + 6) * J->num_sms * b.ox * b.oy);
   }
   const long long mixed = J->dim == 2 && J->fused_ok ? 8ll * J->blk.ngen / std::max(1, J->blk.ntiles) : J->b3_mixed;
-  int dense = 0;
+  int dense = J->b3_slow;
   for (long long c = J->blk.dense; c > 0; c >>= 1) ++dense;
   const std::array<long long, 2> key = {
       ((((((long long)J->dim * 8 + J->g.layout) * 4 + J->g.precision) * 8 + J->vec) * 64 + lg) * 16 + lade) * 8 +
           (J->fused_ok ? 4 : 0) + (J->tma_ok ? 2 : 0) + (J->tma_ok && J->tma.h_ok ? 1 : 0),
-      ((((J->ade_kind + 1ll) * 16 + mixed) * 32 + fill) * 32 + dense) * 4 + (J->ac_host.size() > sizeof(AdeCoef<T>) ? 2 : 0) + (J->block3_ok ? 1 : 0)};
+      (((((J->ade_kind + 1ll) * 16 + mixed) * 32 + fill) * 32 + dense) * 16 + J->b3_src) * 4 + (J->ac_host.size() > sizeof(AdeCoef<T>) ? 2 : 0) + (J->block3_ok ? 1 : 0)};
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     auto it = g_tune.find(key);
@@ -2312,11 +2326,19 @@ int tune_tiles(fdtd_job *J) {
   StepParams<T> p;
   fill_common<T>(J, p);
   p.roles = ROLE_MAIN;
+  // the sources take part, their values zero (256^3 with 16 planes of them: 468 us a
+  // step in the 3D block-step kernel, 275 split)
+  set_sources<T>(J, p);
+  p.n = 1;
+  const size_t zero_bytes = kMaxSrc * kBlockSteps * sizeof(double);
+  void *zeros = nullptr;
+  if (const int rc = alloc_dev(J, &zeros, zero_bytes)) return rc;
+  p.srcval_tab = (const double *)zeros;
   cudaEvent_t a = nullptr, b = nullptr;
   CK(cudaEventCreate(&a));
   CK(cudaEventCreate(&b));
-  float best = 3.0e38f, best_split = 3.0e38f;
-  int choice = 1;
+  float best = 3.0e38f, best_split = 3.0e38f, best_plain = 3.0e38f;
+  int choice = 1, plain_tile = 1;
   // 3D: also the z-marching kernels and, where set up, the TMA-staged cores
   // and the fused step kernel (one launch in place of an E and an H core)
   const int nshapes = J->dim == 3 ? (J->fused_ok ? 9 : J->tma_ok ? (J->tma.h_ok ? 8 : 7) : 6) : J->fused_ok ? 4 : 3;
@@ -2397,18 +2419,24 @@ int tune_tiles(fdtd_job *J) {
     if (c >= nshapes && c < kBlock3Tile) continue;
     const bool block = (J->dim == 2 && c == fused_tile(J)) || (J->dim == 3 && c == kBlock3Tile);
     if (block) {
-      best = time5(split_step);
       // 3D: the fused kernel may be the best core and yet lose with the edges that
-      // it leaves to others (256 x 256 x 128: 178 us a step, the split shape 143)
-      if (J->dim == 3 && choice == fused_tile(J)) {
-        const float fused = best;
-        choice = J->split_tile;
-        best = time5(split_step);
-        if (fused < best) {
-          best = fused;
-          choice = fused_tile(J);
-        }
+      // it leaves to others (256 x 256 x 128: 178 us a step, the split shape 143),
+      // or the other way round (256^3 with sources on every row: 455 and 494, and
+      // 466 with cores that are not TMA-staged)
+      best = 3.0e38f;
+      const int whole[3] = {J->dim == 3 ? J->split_tile : choice, J->split_tile >= 6 ? plain_tile : -1,
+                            J->fused_ok ? fused_tile(J) : -1};
+      int fastest = whole[0];
+      for (int u = 0; u < (J->dim == 3 ? 3 : 1); ++u) {
+        if (whole[u] < 0) continue;
+        choice = whole[u];
+        const float t = time5(split_step);
+        if (t >= best) continue;
+        best = t;
+        fastest = choice;
       }
+      choice = fastest;
+      if (J->dim == 3 && choice < fused_tile(J)) J->split_tile = choice;
     }
     p.tile = c;
     // (the first seven runs or so of the 3D block-step kernel take a quarter longer than all later ones)
@@ -2418,6 +2446,10 @@ int tune_tiles(fdtd_job *J) {
     if (block && failed) {  // a kernel that did not run is no candidate
       cudaGetLastError();
       continue;
+    }
+    if (J->dim == 3 && c < 6 && ms < best_plain) {
+      best_plain = ms;
+      plain_tile = c;
     }
     if (c < fused_tile(J) && ms < best_split) {
       best_split = ms;
@@ -2441,6 +2473,7 @@ int tune_tiles(fdtd_job *J) {
   }
   cudaEventDestroy(a);
   cudaEventDestroy(b);
+  free_dev(J, zeros, zero_bytes);
   CK(cudaGetLastError());
   J->tile = choice;
   if (failed) return FDTD_OK;  // the next job of the kind tries again

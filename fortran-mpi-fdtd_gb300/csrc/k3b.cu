@@ -285,7 +285,25 @@ __global__ void __launch_bounds__(32 * NW, 1) step3d_block(const __grid_constant
   };
   pdl_wait();
   pdl_release();
-  const int n = step_n(p);
+  // the sources' values of the launch's steps, [step][source]: read from the table
+  // per cell and component they made a line of sources along z, one row of one
+  // column of tiles, hold up a launch (256^3: 760 us a step, 260 without it)
+  __shared__ float srcv[2 * kMaxSrc];
+  if (p.nsrc > 0) {
+    const int n = step_n(p);
+    if (threadIdx.x < NS * p.nsrc) srcv[threadIdx.x] = float(p.srcval_tab[(long long)(n - 1) * p.nsrc + threadIdx.x]);
+    __syncthreads();
+  }
+  // their sum on component comp of a cell in step s
+  auto src_at = [&](int s, int comp, int x, int y, int z) {
+    float v = 0.0f;
+    for (int q = 0; q < p.nsrc; ++q) {
+      const Source &sr = p.src[q];
+      if (sr.comp == comp && x >= sr.lo[0] && x <= sr.hi[0] && y >= sr.lo[1] && y <= sr.hi[1] && z >= sr.lo[2] && z <= sr.hi[2])
+        v += srcv[s * p.nsrc + q];
+    }
+    return v;
+  };
 
   // plane k's fields live in one of four slots from its load to its store
   f2 E[4][3] = {}, H[4][3] = {}, nxd = 0, nzd = 0;  // nxd, nzd: Hx, Hz of the row below on the next plane
@@ -480,7 +498,7 @@ __global__ void __launch_bounds__(32 * NW, 1) step3d_block(const __grid_constant
       float x[3], inc[3];
 #pragma unroll
       for (int u = 0; u < 3; ++u) {
-        const float sv = src ? src_sum<float>(p, n + s, u, i + q, j, kw) : 0.0f;
+        const float sv = src ? src_at(s, u, i + q, j, kw) : 0.0f;
         x[u] = q ? hi2(e[u]) : lo2(e[u]);
         const f2 sum = add2(a[u], c[u]);
         inc[u] = fma1(p.ku, q ? hi2(sum) : lo2(sum), sv);
@@ -676,13 +694,18 @@ __global__ void row_flags3_kernel(const __grid_constant__ StepParams<float> p, c
   const int j = (int)(row % p.ny), k = (int)(row / p.ny);
   const bool split = p.pml_mode == 2;
   const bool genz = k < p.mlo[2] || k > p.mhi[2] || (split && (k < p.slo[2] || k > p.shi[2]));
-  bool mix = false, ade = false, gen = genz || j < p.mlo[1] || j > p.mhi[1] || (j == 0 && !p.per[1]) ||
+  const bool rsrc = p.rowflag[row] & ROW_SRC;
+  bool mix = false, ade = false, src = false, gen = genz || j < p.mlo[1] || j > p.mhi[1] || (j == 0 && !p.per[1]) ||
                           (split && (j < p.slo[1] || j > p.shi[1]));
 #pragma unroll
   for (int q = 0; q < 2; ++q) {
     int i = tx * b.ox - 2 + 2 * lane + q;
     if (p.per[0]) i = ((i % p.nx) + p.nx) % p.nx;
     if (i < p.mlo[0] || i > p.mhi[0] || (split && (i < p.slo[0] || i > p.shi[0]))) gen = true;
+    if (rsrc && i >= 0 && i < p.nx)
+      for (int s = 0; s < p.nsrc; ++s)
+        src |= i >= p.src[s].lo[0] && i <= p.src[s].hi[0] && j >= p.src[s].lo[1] && j <= p.src[s].hi[1] &&
+               k >= p.src[s].lo[2] && k <= p.src[s].hi[2];
     if (i >= 0 && i < p.nx) {
       const int id = p.mat[row * p.nx + i];
       mix |= id != p.id0;
@@ -698,11 +721,12 @@ __global__ void row_flags3_kernel(const __grid_constant__ StepParams<float> p, c
   for (int m = lane; m < p.nprobe; m += 32)
     smp |= j == p.probe[m].cell[1] && k == p.probe[m].cell[2] && p.probe[m].cell[0] >= x0 && p.probe[m].cell[0] <= x1;
   mix = __any_sync(0xffffffffu, mix);
+  src = __any_sync(0xffffffffu, src);
   ade = __any_sync(0xffffffffu, ade);
   gen = __any_sync(0xffffffffu, gen);
   smp = __any_sync(0xffffffffu, smp);
   if (lane == 0)
-    out[t] = (uint8_t)((smp ? B3_SMP : 0) | (p.rowflag[row] & B3_SRC) | (mix ? B3_MIX : 0) | (gen ? B3_GEN : 0) | (genz ? B3_GENZ : 0) | (ade ? B3_ADE : 0));
+    out[t] = (uint8_t)((smp ? B3_SMP : 0) | (src ? B3_SRC : 0) | (mix ? B3_MIX : 0) | (gen ? B3_GEN : 0) | (genz ? B3_GENZ : 0) | (ade ? B3_ADE : 0));
 }
 
 constexpr int kB3Warps = 16;
