@@ -260,6 +260,7 @@ struct fdtd_job {
   // leave out kernels that need second sets of buffers: 1 the block-step kernels,
   // but for the TMz jobs that have such a set for any kernel of whole steps; 2 all
   int lean = 0;
+  bool shared = false;  // a server may run it beside other jobs
   Block3 b3{};
   void *spb3[6] = {};
   size_t b3_bytes[6] = {};  // of the flags, slot map, first step's dispersive state, its sampled rows, order, segments
@@ -2312,7 +2313,8 @@ int tune_tiles(fdtd_job *J) {
   const std::array<long long, 2> key = {
       ((((((long long)J->dim * 8 + J->g.layout) * 4 + J->g.precision) * 8 + J->vec) * 64 + lg) * 16 + lade) * 8 +
           (J->fused_ok ? 4 : 0) + (J->tma_ok ? 2 : 0) + (J->tma_ok && J->tma.h_ok ? 1 : 0),
-      (((((J->ade_kind + 1ll) * 16 + mixed) * 32 + fill) * 32 + dense) * 16 + J->b3_src) * 4 + (J->ac_host.size() > sizeof(AdeCoef<T>) ? 2 : 0) + (J->block3_ok ? 1 : 0)};
+      (((((J->ade_kind + 1ll) * 16 + mixed) * 32 + fill) * 32 + dense) * 16 + J->b3_src) * 8 + (J->shared ? 4 : 0) +
+          (J->ac_host.size() > sizeof(AdeCoef<T>) ? 2 : 0) + (J->block3_ok ? 1 : 0)};
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     auto it = g_tune.find(key);
@@ -2334,9 +2336,10 @@ int tune_tiles(fdtd_job *J) {
   void *zeros = nullptr;
   if (const int rc = alloc_dev(J, &zeros, zero_bytes)) return rc;
   p.srcval_tab = (const double *)zeros;
-  cudaEvent_t a = nullptr, b = nullptr;
+  cudaEvent_t a = nullptr, b = nullptr, c2 = nullptr;
   CK(cudaEventCreate(&a));
   CK(cudaEventCreate(&b));
+  CK(cudaEventCreate(&c2));
   float best = 3.0e38f, best_split = 3.0e38f, best_plain = 3.0e38f;
   int choice = 1, plain_tile = 1;
   // 3D: also the z-marching kernels and, where set up, the TMA-staged cores
@@ -2401,18 +2404,24 @@ int tune_tiles(fdtd_job *J) {
     launch_part<T>(J, p, K2D_CORE, true, J->stream);
     launch_part<T>(J, p, K2D_CORE, false, J->stream);
   };
-  // the time of five runs, from two where they are long and even: of large grids,
-  // and of the 2D block-step kernel's eight steps
+  // the time of five runs; where they are long, of large grids and of the 2D
+  // block-step kernel's eight steps, from the shorter of two (other jobs of a
+  // server may run beside them)
   const bool large = J->ncell >= (J->dim == 3 ? 4000000 : 16000000);
   auto time5 = [&](auto run, bool few = false) {
     few |= large;
     for (int w = 0; w < (few ? 1 : 2); ++w) run();
     cudaEventRecord(a, J->stream);
-    for (int r = 0; r < (few ? 2 : 5); ++r) run();
+    for (int r = 0; r < (few ? 1 : 5); ++r) run();
     cudaEventRecord(b, J->stream);
-    float ms = 0.f;
-    if (cudaEventSynchronize(b) != cudaSuccess || cudaEventElapsedTime(&ms, a, b) != cudaSuccess) return 3.0e38f;
-    return few ? 2.5f * ms : ms;
+    if (few) {
+      run();
+      cudaEventRecord(c2, J->stream);
+    }
+    float ms = 0.f, ms2 = 3.0e38f;
+    if (cudaEventSynchronize(few ? c2 : b) != cudaSuccess || cudaEventElapsedTime(&ms, a, b) != cudaSuccess) return 3.0e38f;
+    if (few && cudaEventElapsedTime(&ms2, b, c2) != cudaSuccess) return 3.0e38f;
+    return few ? 5.0f * std::min(ms, ms2) : ms;
   };
   const int last = J->block3_ok ? kBlock3Tile : nshapes - 1;
   for (int c = 0; c <= last; ++c) {
@@ -2464,15 +2473,19 @@ int tune_tiles(fdtd_job *J) {
     if (block && J->dim == 2)
       for (J->block_min = 1; J->block_min < pl.ks && ms * pl.ks * (0.5f + J->block_min / 16.f) > J->block_min * (best + 0.015f);)
         ++J->block_min;
-    // (in a replayed graph a split step is a few per cent shorter than here: 200^3
-    // 142 us, where the 3D block-step kernel takes 145)
-    if (ms * (J->dim == 3 && block ? 1.05f : 1.0f) < best) {
+    // (In a replayed graph a split step is a few per cent shorter than here: 200^3
+    // 142 us, where the 3D block-step kernel takes 145.  Beside other jobs that
+    // kernel's half of the memory traffic counts for more than its own time: eight
+    // served spheres of 128^3 to 256^3 took 5.95 s with it, 6.30 with the split
+    // shape at 192^3, where it takes 177 us a step alone and the other 132.)
+    if (ms * (J->dim == 3 && block ? (J->shared ? 0.72f : 1.05f) : 1.0f) < best) {
       best = ms;
       choice = c;
     }
   }
   cudaEventDestroy(a);
   cudaEventDestroy(b);
+  cudaEventDestroy(c2);
   free_dev(J, zeros, zero_bytes);
   CK(cudaGetLastError());
   J->tile = choice;
@@ -3402,6 +3415,7 @@ int fdtd::pack_run(fdtd::Pack *P, int rings, cudaEvent_t done) {
 }
 
 // =========================================================================
+void fdtd::make_shared(fdtd_job *J) { J->shared = true; }
 void fdtd::make_lean(fdtd_job *J, int level) { J->lean = level; }
 
 uint64_t fdtd::lean_estimate(fdtd_job *J, int level) {

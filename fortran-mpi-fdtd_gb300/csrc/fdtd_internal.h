@@ -406,6 +406,8 @@ struct DftParams {
 // 1: the block-step kernels; 2: the fused ones too), and the estimate it then has
 // (fdtd_server.cu: a job that does not fit with them)
 void make_lean(fdtd_job *job, int level);
+// an uncommitted job of a server that runs several at a time
+void make_shared(fdtd_job *job);
 uint64_t lean_estimate(fdtd_job *job, int level);
 template <typename T> void launch_dft(const DftParams &d, const T *stage, void *stream);
 // every ring of a line's stage in one launch, for monitors of few samples

@@ -393,6 +393,7 @@ int fdtd_server_submit(fdtd_server *S, fdtd_job *job, int32_t n_steps, int64_t *
   if (rc) return rc;
   Req *r = new Req;
   r->job = job;
+  if (S->d.max_active > 1) fdtd::make_shared(job);
   r->n_steps = n_steps;
   r->est = est;
   r->t_submit = now_s();
