@@ -114,8 +114,8 @@ def test_failed_launch_is_an_error_and_no_step(gpu, monkeypatch, dim):
 
 
 def test_kernel_that_fails_in_the_tuner_is_left_out(gpu):
-    spec, _ = problems.config_2d_tmz(precision=abi.F32, n=160, ncyl=1, nfreq=6, npml=12)
-    spec.materials = spec.materials[:1]  # a kind of grid of its own, not timed yet in this process
+    spec, _ = problems.config_2d_tmz(precision=abi.F32, n=163, ncyl=1, nfreq=6, npml=12)
+    spec.materials = spec.materials[:1]  # odd rows of vacuum: a kind of grid that no other test has timed in this process
     try:
         gpu.fail_launch_after(0)
         J = gpu.Job(spec)
@@ -123,7 +123,8 @@ def test_kernel_that_fails_in_the_tuner_is_left_out(gpu):
         gpu.fail_launch_after(-1)
     assert J.tile() in (1, 2, 3)
     J.step(1, 200)
-    K = gpu.Job(spec, tile=4)
+    K = gpu.Job(spec)  # the failure is not kept: the kernel is a candidate again
+    assert K.tile() == 4
     K.step(1, 200)
     for a, b in zip(state_of(J, FIELDS_TM), state_of(K, FIELDS_TM)):
         np.testing.assert_array_equal(a, b)
